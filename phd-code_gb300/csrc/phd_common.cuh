@@ -2,6 +2,7 @@
 #pragma once
 #include <atomic>
 #include <cstdint>
+#include <utility>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 #include "../../include/phdflux.h"
@@ -33,6 +34,26 @@ struct NvtxRange {
 // Launched without the attribute, both are no-ops in effect.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+#ifdef __CUDACC__
+// A kernel launched with programmatic stream serialization: it may be scheduled while the
+// previous kernel of the stream drains (the kernels wait for it with pdl_wait before
+// reading what it writes).  Captured into CUDA graphs as programmatic edges.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+#endif
 
 // Threads per block for a launch over n items with at most max_block threads: halved
 // (down to one warp) while the grid would not cover every SM twice, so small meshes

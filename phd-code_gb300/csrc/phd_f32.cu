@@ -1108,25 +1108,6 @@ int cells_prim_f32(const phd_mesh *mesh, const phd_params *par, const phd_geom32
     return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
 }
 
-// A step kernel launched with programmatic stream serialization: it may be scheduled
-// while the previous kernel of the stream drains (the kernels wait for it with
-// pdl_wait before reading what it writes).  Captured into CUDA graphs as programmatic
-// edges.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
 template <int SOLVER, int ITEMS>
 void launch_face32_items(bool linear, int grid, int block, cudaStream_t s, const phd_mesh &M, const phd_params &P,
                          int moving, const phd_geom32 *G, const float4 *prim4, const float4 *cellrec, const float2 *w2,

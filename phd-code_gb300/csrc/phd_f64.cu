@@ -6,6 +6,7 @@
 #include "phd_common.cuh"
 #include "phd_physics.cuh"
 #include "phd_ref.cuh"
+#include "phd_fp64.cuh"
 
 namespace phd {
 
@@ -154,30 +155,293 @@ __device__ int cell_gradient_f64(const phd_mesh &M, const double *__restrict__ p
     return status;
 }
 
-// Real rows: own gradient.  Ghost rows: the image's gradient (computed again from the
-// image's faces, bit-identical), with the reflective diagonal flip of grad v
-// (domain_manager.pyx:819-835, boundary.pyx:287-307).
-template <int DIM, bool TAPE = false>
-__global__ void __launch_bounds__(BLOCK) k_gradients(phd_mesh M, const double *__restrict__ prim,
-                                                      int limiter, double *__restrict__ grad,
-                                                      phd_clock *clk, GradTape tape = GradTape{nullptr, nullptr}) {
-    constexpr int NF = DIM + 2;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M.n_cells) return;
-    int c = i;
-    if (M.tag[i] != PHD_REAL_TAG) {
-        c = M.map[i];
-        if (c < 0 || c >= M.n_cells) { set_status(clk, PHD_STATUS_BAD_INDEX); return; }
+// One row of the gradient on the plain path: a real cell's own gradient, a ghost's its
+// image's (computed again from the image's faces, bit-identical) with the reflective
+// diagonal flip of grad v (domain_manager.pyx:819-835, boundary.pyx:287-307).
+template <bool TAPE>
+__device__ __noinline__ int gradient_row_plain(const phd_mesh *M, const double *prim, int limiter, int i, int c,
+                                               double *grad, GradTape tape) {
+    double df[8];
+    const int st = cell_gradient_f64<2, TAPE>(*M, prim, limiter, c, df, tape, i == c);
+    const int fl = M->flip ? M->flip[i] : 0;
+    if (fl & 1) df[2] *= -1;
+    if (fl & 2) df[5] *= -1;
+#pragma unroll
+    for (int r = 0; r < 8; r++) grad[(size_t)r * M->n_cells + i] = df[r];
+    return st;
+}
+
+// Limited gradients of NC rows (cells) by 4 NC threads, the same numbers as cell_gradient_f64
+// bit for bit.  The kernel is bound by the FP64 pipe (phd_fp64.cuh), so the work is laid
+// out for few and full FP64 warp instructions:
+//  * per face of the block, one thread forms the face's terms of the Green-Gauss sum for
+//    both of its cells: the numerators area (d_dif c - d_sum dr / 2) differ only in sign
+//    between the two sides, the quotients by r V take one seed a side.  (A thread a cell
+//    formed every numerator twice, and its warp ran as long as its longest list: 20 of 32
+//    lanes active.)  Where the other cell lies outside the block its side is left out, and
+//    such faces are kept apart from the others so that their warps skip it too;
+//  * the terms go to shared memory by list entry; a thread a cell and field adds them in list
+//    order, finds the neighbours' extrema by integer comparison and limits;
+//  * the AREPO limiter's minimum over faces of (phi_ext - phi)/dphi is reached at the
+//    largest |dphi| of either sign, the numerator being common and rounding monotonic: two
+//    quotients a field instead of one a face, and none where it would be at least 1.
+// A block that meets anything unusual -- an index out of range, a cell that its face does not
+// name, more list entries than the shared arrays hold, an operand outside the seeds' windows
+// -- does its rows on the plain path, status bits included.
+template <int NC>
+struct GradShared {
+    static constexpr int CAP = 8 * NC;              // list entries: six a cell on average
+    double q[8][CAP], sep[2][CAP], pj[4][CAP];
+    int fid[CAP], other[CAP];
+    unsigned char slot[CAP];
+    int task[2][CAP];                               // two-sided from the front, one-sided
+    int cell[NC], c[NC], off[NC + 1], ptr[NC], nreal[NC];
+    int ntask[2], odd;
+    double res_v[4][NC];                            // TESS: each field's minimum, and where
+    int res_e[4][NC];
+};
+
+// The entry of the block's row t whose face is fid (its first), or -1.
+template <int NC>
+__device__ __forceinline__ int find_entry(const GradShared<NC> &S, int t, int fid) {
+    for (int k = S.off[t]; k < S.off[t + 1]; k++)
+        if (S.fid[k] == fid) return k;
+    return -1;
+}
+
+template <int NC, bool TAPE>
+__global__ void __launch_bounds__(4 * NC) k_gradients(const __grid_constant__ phd_mesh M, const double *__restrict__ prim, int limiter,
+                                                      double *__restrict__ grad, phd_clock *clk,
+                                                      GradTape tape = GradTape{nullptr, nullptr}) {
+    __shared__ GradShared<NC> S;
+    const int n = M.n_cells, F = M.n_faces, tid = threadIdx.x, c0 = blockIdx.x * NC;
+    pdl_launch_dependents();
+    pdl_wait();                                      // prim: written by the previous step's update
+    if (tid == 0) { S.ntask[0] = S.ntask[1] = 0; S.odd = 0; }
+    // rows, their source cells and list bounds
+    if (tid < NC) {
+        const int i = c0 + tid;
+        int c = -1, real = 0, e0 = 0, len = 0;
+        if (i < n) {
+            real = M.tag[i] == PHD_REAL_TAG;
+            c = real ? i : M.map[i];
+            if (c < 0 || c >= n) c = -1;
+            else {
+                e0 = M.nbr_ptr[c];
+                len = M.nbr_ptr[c + 1] - e0;
+            }
+        }
+        S.c[tid] = c;
+        S.nreal[tid] = real;
+        S.ptr[tid] = e0;
+        S.cell[tid] = len;
     }
-    double df[NF * DIM];
-    const int st = cell_gradient_f64<DIM, TAPE>(M, prim, limiter, c, df, tape, i == c);
-    set_status(clk, st);
+    __syncthreads();
+    if (tid < 32) {                                  // exclusive scan of the lengths
+        int run = 0;
+#pragma unroll
+        for (int b = 0; b < NC; b += 32) {
+            const int len = S.cell[b + tid];
+            int inc = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, inc, o);
+                if (tid >= o) inc += t;
+            }
+            S.off[b + tid] = run + inc - len;
+            if (len < 0) S.odd = 1;
+            run += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (tid == 0) {
+            S.off[NC] = run;
+            if (run > GradShared<NC>::CAP) S.odd = 1;
+        }
+    }
+    __syncthreads();
+    const int E = S.off[NC];
+    bool ok = true;
+    if (!S.odd) {
+        for (int k = tid; k < E; k += 4 * NC) {
+            int lo = 0, hi = NC;                     // off[lo] <= k < off[hi]
+#pragma unroll
+            for (int s = NC; s > 1; s >>= 1) {
+                const int mid = (lo + hi) >> 1;
+                if (S.off[mid] <= k) lo = mid;
+                else hi = mid;
+            }
+            S.slot[k] = (unsigned char)lo;
+            S.fid[k] = M.nbr_idx[S.ptr[lo] + (k - S.off[lo])];
+        }
+    }
+    __syncthreads();
+    if (!S.odd) {
+        for (int k = tid; k < E; k += 4 * NC) {
+            const int s = S.slot[k], c = S.c[s], fid = S.fid[k];
+            int a = -1, b = -1;
+            if (fid >= 0 && fid < F) {
+                a = M.pair_i[fid];
+                b = M.pair_j[fid];
+            }
+            const int j = (c == a) ? b : a;
+            if ((c != a && c != b) || j < 0 || j >= n) { ok = false; continue; }
+            S.other[k] = j;
+            const int t = j - c0;                    // the other cell's row, when it is in this block
+            int k2 = -1;
+            if (j != c && t >= 0 && t < NC && S.nreal[t] && S.nreal[s]) k2 = find_entry(S, t, fid);
+            if (k2 >= 0) {
+                if (c == a) S.task[0][atomicAdd(&S.ntask[0], 1)] = k | (k2 << 16);
+                else if (find_entry(S, s, fid) != k) ok = false;        // the same face twice in a list
+            } else {
+                S.task[1][atomicAdd(&S.ntask[1], 1)] = k;
+            }
+        }
+        if (!ok) S.odd = 1;
+    }
+    __syncthreads();
+    if (!S.odd) {
+        const int n2 = S.ntask[0], nt = n2 + S.ntask[1];
+        for (int t = tid; t < nt; t += 4 * NC) {
+            const int code = t < n2 ? S.task[0][t] : S.task[1][t - n2];
+            const bool two = t < n2;
+            const int k = code & 0xffff, k2 = code >> 16;
+            const int c = S.c[S.slot[k]], j = S.other[k], fid = S.fid[k];
+            const double xc = M.x[c], yc = M.x[(size_t)n + c], xj = M.x[j], yj = M.x[(size_t)n + j];
+            const double comx = M.com[fid], comy = M.com[(size_t)F + fid], area = M.area[fid];
+            const double cfx = fma(-0.5, xc + xj, comx), cfy = fma(-0.5, yc + yj, comy);
+            const double drx = xc - xj, dry = yc - yj;
+            const double r = f64_sqrt(drx * drx + dry * dry, ok);
+            const double rc = r * M.vol[c], rj = two ? r * M.vol[j] : 1.0;
+            const double ic = f64_rcp(rc, ok), ij = f64_rcp(rj, ok);
+            S.sep[0][k] = comx - (xc + M.dcom[c]);
+            S.sep[1][k] = comy - (yc + M.dcom[(size_t)n + c]);
+            if (two) {
+                S.sep[0][k2] = comx - (xj + M.dcom[j]);
+                S.sep[1][k2] = comy - (yj + M.dcom[(size_t)n + j]);
+            }
+#pragma unroll
+            for (int f = 0; f < 4; f++) {
+                const double pc = prim[(size_t)f * n + c], pj = prim[(size_t)f * n + j];
+                const double d_dif = pj - pc, d_sum = pj + pc;
+                const double nx = area * fma(-0.5, d_sum * drx, d_dif * cfx);
+                const double ny = area * fma(-0.5, d_sum * dry, d_dif * cfy);
+                S.q[2 * f][k] = f64_div_by(nx, rc, ic, ok);
+                S.q[2 * f + 1][k] = f64_div_by(ny, rc, ic, ok);
+                S.pj[f][k] = pj;
+                if (two) {
+                    S.q[2 * f][k2] = -f64_div_by(nx, rj, ij, ok);
+                    S.q[2 * f + 1][k2] = -f64_div_by(ny, rj, ij, ok);
+                    S.pj[f][k2] = pc;
+                }
+            }
+        }
+        if (!ok) S.odd = 1;
+    }
+    __syncthreads();
+    const int s = tid % NC, f = tid / NC, i = c0 + s;
+    const int c = S.c[s];
+    double gx = 0., gy = 0., alpha = 1.0;
+    int act = -1, emax = -1, emin = -1;
+    if (!S.odd && c >= 0) {
+        const double pc = prim[(size_t)f * n + c];
+        const int k0 = S.off[s], k1 = S.off[s + 1];
+        double pmax = pc, pmin = pc;
+        long long kmax = f64_key(pc), kmin = kmax;
+        for (int k = k0; k < k1; k++) {
+            gx = gx + S.q[2 * f][k];
+            gy = gy + S.q[2 * f + 1][k];
+            const double pj = S.pj[f][k];
+            const long long kp = f64_key(pj);
+            if (kp > kmax) { kmax = kp; pmax = pj; emax = k; }
+            if (kp < kmin) { kmin = kp; pmin = pj; emin = k; }
+        }
+        if (limiter == PHD_LIMITER_AREPO) {
+            double hi = 0., lo = 0.;
+            int ehi = -1, elo = -1;
+            for (int k = k0; k < k1; k++) {
+                const double dphi = gx * S.sep[0][k] + gy * S.sep[1][k];
+                if (f64_lt(hi, dphi)) { hi = dphi; ehi = k; }
+                if (f64_lt(dphi, lo)) { lo = dphi; elo = k; }
+            }
+            const double up = pmax - pc, dn = pmin - pc;
+            double ph = 1.0, pl = 1.0;
+            if (f64_lt(up, hi)) ph = f64_div(up, hi, ok);
+            if (f64_lt(lo, dn)) pl = f64_div(dn, lo, ok);
+            ph = f64_max(ph, 0.);
+            pl = f64_max(pl, 0.);
+            alpha = f64_min(f64_min(ph, pl), 1.0);
+            if (TAPE && f64_lt(alpha, 1.0)) {
+                // the first entry in list order that reaches the minimum
+                int e = f64_lt(pl, ph) ? elo : ehi;
+                if (f64_key(ph) == f64_key(pl)) e = min(ehi, elo);
+                act = f64_pos(alpha) ? e : -2;
+            }
+        } else if (limiter == PHD_LIMITER_TESS) {
+            for (int k = k0; k < k1; k++) {
+                const double dphi = gx * S.sep[0][k] + gy * S.sep[1][k], num = S.pj[f][k] - pc;
+                if (f64_zero(dphi)) continue;                            // psi = 1
+                double psi = 0.;                                         // opposite signs, or a flat neighbour
+                if (!f64_zero(num) && (f64_bits(num) ^ f64_bits(dphi)) >= 0) {
+                    const long long m = 0x7fffffffffffffffll;
+                    if ((f64_bits(num) & m) >= (f64_bits(dphi) & m)) continue;       // psi >= 1
+                    psi = f64_div(num, dphi, ok);
+                }
+                if (f64_lt(psi, alpha)) { alpha = psi; act = k; }
+            }
+            S.res_v[f][s] = alpha;
+            S.res_e[f][s] = act;
+        }
+        if (!ok) S.odd = 1;
+    }
+    __syncthreads();
+    if (S.odd) {                                     // uniform over the block
+        if (tid < NC && i < n) {
+            if (c < 0) set_status(clk, PHD_STATUS_BAD_INDEX);
+            else set_status(clk, gradient_row_plain<TAPE>(&M, prim, limiter, i, c, grad, tape));
+        }
+        return;
+    }
+    if (i >= n) return;
+    if (c < 0) {
+        if (f == 0) set_status(clk, PHD_STATUS_BAD_INDEX);
+        return;
+    }
+    int act_f0 = -1;
+    if (limiter == PHD_LIMITER_TESS) {
+        // every field limits the density's slope alone (reconstruction.pyx:731); the minimum
+        // over faces and fields, the first in that order
+        alpha = 1.0;
+        act = -1;
+        if (f == 0) {
+            int e = -1;
+#pragma unroll
+            for (int g = 0; g < 4; g++) {
+                const double v = S.res_v[g][s];
+                const int ke = S.res_e[g][s];
+                if (ke >= 0 && (f64_lt(v, alpha) || (f64_key(v) == f64_key(alpha) && e >= 0 && ke < e))) {
+                    alpha = v;
+                    e = ke;
+                    act_f0 = g;
+                }
+            }
+            if (TAPE) act = e < 0 ? -1 : (f64_pos(alpha) ? e : -2);
+        }
+    }
+    if (TAPE && i == c) {
+        const int g0 = S.ptr[s] - S.off[s];          // entry of the block -> list entry
+        tape.f64[(size_t)(2 * f) * n + i] = gx;
+        tape.f64[(size_t)(2 * f + 1) * n + i] = gy;
+        tape.f64[(size_t)(8 + f) * n + i] = alpha;
+        tape.i32[(size_t)f * n + i] = act >= 0 ? act + g0 : act;
+        tape.i32[(size_t)(4 + f) * n + i] = emax >= 0 ? emax + g0 : -1;
+        tape.i32[(size_t)(8 + f) * n + i] = emin >= 0 ? emin + g0 : -1;
+        if (f == 0) tape.i32[(size_t)12 * n + i] = act_f0;
+    }
     const int fl = M.flip ? M.flip[i] : 0;
-#pragma unroll
-    for (int kk = 0; kk < DIM; kk++)
-        if (fl & (1 << kk)) df[DIM * (1 + kk) + kk] *= -1;
-#pragma unroll
-    for (int r = 0; r < NF * DIM; r++) grad[(size_t)r * M.n_cells + i] = df[r];
+    double ox = alpha * gx, oy = alpha * gy;
+    if (f == 1 && (fl & 1)) ox = -ox;
+    if (f == 2 && (fl & 2)) oy = -oy;
+    grad[(size_t)(2 * f) * n + i] = ox;
+    grad[(size_t)(2 * f + 1) * n + i] = oy;
 }
 
 template <int DIM>
@@ -543,6 +807,15 @@ __global__ void __launch_bounds__(BLOCK) k_face_vel(phd_mesh M, const double *__
 inline int blk_of(int n) { return block_for(n, BLOCK); }
 inline int grid_of(int n) { return grid_for_block(n, blk_of(n)); }
 
+// Gradients of n rows: blocks of 32 rows (128 threads).
+inline void launch_gradients(const phd_mesh &M, const double *prim, int limiter, double *grad, phd_clock *clk,
+                             GradTape tape, cudaStream_t stream) {
+    constexpr int NC = 32;
+    const int grid = (M.n_cells + NC - 1) / NC;
+    if (tape.f64) launch_pdl(k_gradients<NC, true>, grid, 4 * NC, stream, M, prim, (int)limiter, grad, clk, tape);
+    else launch_pdl(k_gradients<NC, false>, grid, 4 * NC, stream, M, prim, (int)limiter, grad, clk, tape);
+}
+
 inline int launch_status() {
     return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
 }
@@ -574,15 +847,14 @@ const char *phd_status_string(int bit) {
 int phd_gradients_f64(const phd_mesh *mesh, const double *prim, int32_t limiter, double *grad,
                       phd_clock *clk, cudaStream_t stream) {
     if (!mesh_ok(mesh) || !prim || !grad) return PHD_ERR_ARG;
-    k_gradients<2><<<grid_of(mesh->n_cells), blk_of(mesh->n_cells), 0, stream>>>(*mesh, prim, limiter, grad, clk);
+    launch_gradients(*mesh, prim, limiter, grad, clk, GradTape{nullptr, nullptr}, stream);
     return launch_status();
 }
 
 int phd_gradients_f64_taped(const phd_mesh *mesh, const double *prim, int32_t limiter, double *grad,
                             double *tape_f64, int32_t *tape_i32, phd_clock *clk, cudaStream_t stream) {
     if (!mesh_ok(mesh) || !prim || !grad || !tape_f64 || !tape_i32) return PHD_ERR_ARG;
-    k_gradients<2, true><<<grid_of(mesh->n_cells), blk_of(mesh->n_cells), 0, stream>>>(
-        *mesh, prim, limiter, grad, clk, GradTape{tape_f64, tape_i32});
+    launch_gradients(*mesh, prim, limiter, grad, clk, GradTape{tape_f64, tape_i32}, stream);
     return launch_status();
 }
 
@@ -695,10 +967,7 @@ static int step_f64(const phd_mesh *mesh, const phd_params *par, int32_t moving,
         k_gen_vel<2><<<gc, bc, 0, stream>>>(*mesh, prim, par->gamma, par->eta, par->regularize, w);
         if (mesh->n_faces) k_face_vel<2><<<gf, bf, 0, stream>>>(*mesh, w, face_w);
     }
-    if (linear) {
-        if (tape.f64) k_gradients<2, true><<<gc, bc, 0, stream>>>(*mesh, prim, par->limiter, grad, clk, tape);
-        else k_gradients<2><<<gc, bc, 0, stream>>>(*mesh, prim, par->limiter, grad, clk);
-    }
+    if (linear) launch_gradients(*mesh, prim, par->limiter, grad, clk, tape, stream);
     if (marks) cudaEventRecord(marks[1], stream);
     if (mesh->n_faces)
         k_face_flux<2><<<gf, bf, 0, stream>>>(*mesh, *par, prim, grad, face_w, flux, clk);

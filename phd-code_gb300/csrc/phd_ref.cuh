@@ -6,7 +6,7 @@ namespace phd {
 
 // add_spatial reconstruction.pyx:832-921 for face m (reference geometry in FP64).
 template <int DIM>
-__device__ __forceinline__ void face_spatial_f64(const phd_mesh &M, int m, int i, int j, const double *pi,
+PHD_HD __forceinline__ void face_spatial_f64(const phd_mesh &M, int m, int i, int j, const double *pi,
                                                  const double *pj, const double *gi, const double *gj,
                                                  const double *w, bool boost, bool gizmo, double *L,
                                                  double *R) {
