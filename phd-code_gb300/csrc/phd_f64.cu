@@ -6,7 +6,7 @@
 #include "phd_common.cuh"
 #include "phd_physics.cuh"
 #include "phd_ref.cuh"
-#include "phd_fp64.cuh"
+#include "phd_face64.cuh"
 
 namespace phd {
 
@@ -537,31 +537,127 @@ __global__ void __launch_bounds__(BLOCK) k_riemann(phd_mesh M, int solver, doubl
     for (int q = 0; q < NF; q++) flux[(size_t)q * F + m] = f[q];
 }
 
-// Fused: states + Riemann + deboost per face; the states never reach memory.
-template <int DIM>
-__global__ void __launch_bounds__(BLOCK) k_face_flux(phd_mesh M, phd_params P, const double *__restrict__ prim,
-                                                      const double *__restrict__ grad,
-                                                      const double *__restrict__ face_w,
-                                                      double *__restrict__ flux, phd_clock *clk) {
-    constexpr int NF = DIM + 2;
+// assign_face_velocities mesh.pyx:462-477 for one face from its cells' generator velocities.
+__device__ __forceinline__ void face_velocity_plain(const phd_mesh &M, int m, int i, int j, const double *wi,
+                                                    const double *wj, double *fw) {
+    const int n = M.n_cells, F = M.n_faces;
+    double factor = 0.0, denom = 0.0;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double xi = M.x[(size_t)k * n + i], xj = M.x[(size_t)k * n + j];
+        factor = factor + ((wi[k] - wj[k]) * (M.com[(size_t)k * F + m] - (0.5 * (xi + xj))));
+        denom = denom + t_sq(xj - xi);
+    }
+    factor = factor / denom;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double xi = M.x[(size_t)k * n + i], xj = M.x[(size_t)k * n + j];
+        fw[k] = (0.5 * (wi[k] + wj[k])) + (factor * (xj - xi));
+    }
+}
+
+// One face on the plain path; returns status bits.  w (moving): the generator velocities.
+__device__ __noinline__ int face_flux_plain(const phd_mesh *M, const phd_params *P, const double *prim,
+                                            const double *grad, const double *w, double *face_w, double dt_half,
+                                            int m, int i, int j, double *flux) {
+    const int n = M->n_cells, F = M->n_faces;
+    const bool boost = (P->solver == PHD_EXACT) ? true : (P->boost != 0);
+    const bool linear = P->reconstruction == PHD_LINEAR;
+    double pi[4], pj[4], gi[8], gj[8], fw[2], L[4], R[4], nrm[2], f[4];
+    if (w) {
+        const double wi[2] = {w[i], w[(size_t)n + i]}, wj[2] = {w[j], w[(size_t)n + j]};
+        face_velocity_plain(*M, m, i, j, wi, wj, fw);
+        face_w[m] = fw[0];
+        face_w[(size_t)F + m] = fw[1];
+    }
+    load_face_inputs<2>(*M, prim, grad, face_w, m, i, j, linear, pi, pj, gi, gj, fw);
+    face_states_f64<2>(*M, m, i, j, pi, pj, gi, gj, fw, P->gamma, dt_half, boost, linear, P->gizmo != 0, L, R);
+#pragma unroll
+    for (int k = 0; k < 2; k++) nrm[k] = M->normal[(size_t)k * F + m];
+    bool failed = false;
+    riemann_flux<double, 2>(P->solver, L, R, nrm, fw, P->gamma, boost, P->exact_max_iter, f, &failed);
+#pragma unroll
+    for (int q = 0; q < 4; q++) flux[(size_t)q * F + m] = f[q];
+    return failed ? PHD_STATUS_RIEMANN_NONCONVERGED : 0;
+}
+
+// Fused: (moving) face velocity, states, Riemann flux and deboost per face; the states never
+// reach memory.  Bound by the FP64 pipe: see phd_face64.cuh for how the same numbers come
+// out of a third of the FP64 instructions.  The plain path stands in for a face with
+// unusual operands.  128 threads at 128 registers: 16 warps a SM, four times what keeps the
+// FP64 pipe fed.  Measured (160,000 cells, shear layer, HLLC): 1032 us and 35 us for the face
+// velocities by themselves -> 359 us, 1106 + 33 -> 390 FP64 instructions per warp.
+template <int SOLVER>
+__global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ phd_mesh M, const __grid_constant__ phd_params P,
+                                                   const __grid_constant__ Gas64 C, const double *__restrict__ prim,
+                                                   const double *__restrict__ grad, const double *__restrict__ w,
+                                                   double *__restrict__ face_w, double *__restrict__ flux,
+                                                   phd_clock *clk) {
+    pdl_launch_dependents();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M.n_faces) return;
-    const int F = M.n_faces;
+    const int n = M.n_cells, F = M.n_faces;
+    pdl_wait();                                      // prim, grad, w and the clock: earlier kernels'
+    if (m >= F) return;
     const int i = M.pair_i[m], j = M.pair_j[m];
-    if (i < 0 || i >= M.n_cells || j < 0 || j >= M.n_cells) { set_status(clk, PHD_STATUS_BAD_INDEX); return; }
-    const bool boost = (P.solver == PHD_EXACT) ? true : (P.boost != 0);
+    if (i < 0 || i >= n || j < 0 || j >= n) { set_status(clk, PHD_STATUS_BAD_INDEX); return; }
+    const bool boost = SOLVER == PHD_EXACT || P.boost != 0;
     const bool linear = P.reconstruction == PHD_LINEAR;
     const double dt_half = 0.5 * clk->dt;
-    double pi[NF], pj[NF], gi[NF * DIM], gj[NF * DIM], w[DIM], L[NF], R[NF], nrm[DIM], f[NF];
-    load_face_inputs<DIM>(M, prim, grad, face_w, m, i, j, linear, pi, pj, gi, gj, w);
-    face_states_f64<DIM>(M, m, i, j, pi, pj, gi, gj, w, P.gamma, dt_half, boost, linear, P.gizmo != 0, L, R);
+    Face64 A;
 #pragma unroll
-    for (int k = 0; k < DIM; k++) nrm[k] = M.normal[(size_t)k * F + m];
-    bool failed = false;
-    riemann_flux<double, DIM>(P.solver, L, R, nrm, w, P.gamma, boost, P.exact_max_iter, f, &failed);
-    if (failed) set_status(clk, PHD_STATUS_RIEMANN_NONCONVERGED);
+    for (int k = 0; k < 2; k++) {
+        A.xi[k] = M.x[(size_t)k * n + i];
+        A.xj[k] = M.x[(size_t)k * n + j];
+        A.com[k] = M.com[(size_t)k * F + m];
+    }
 #pragma unroll
-    for (int q = 0; q < NF; q++) flux[(size_t)q * F + m] = f[q];
+    for (int f = 0; f < 4; f++) { A.pi[f] = prim[(size_t)f * n + i]; A.pj[f] = prim[(size_t)f * n + j]; }
+    if (linear) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) { A.gi[r] = grad[(size_t)r * n + i]; A.gj[r] = grad[(size_t)r * n + j]; }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            A.ci[k] = M.dcom[(size_t)k * n + i];
+            A.cj[k] = M.dcom[(size_t)k * n + j];
+        }
+    }
+    bool ok = true;
+    if (w) {
+        const double wi[2] = {w[i], w[(size_t)n + i]}, wj[2] = {w[j], w[(size_t)n + j]};
+        const double dx = A.xj[0] - A.xi[0], dy = A.xj[1] - A.xi[1];
+        const double num = (wi[0] - wj[0]) * fma(-0.5, A.xi[0] + A.xj[0], A.com[0]) +
+                           (wi[1] - wj[1]) * fma(-0.5, A.xi[1] + A.xj[1], A.com[1]);
+        const double fac = f64_div(num, dx * dx + dy * dy, ok);
+        A.w[0] = fma(0.5, wi[0] + wj[0], fac * dx);
+        A.w[1] = fma(0.5, wi[1] + wj[1], fac * dy);
+    } else {
+        A.w[0] = face_w ? face_w[m] : 0.0;
+        A.w[1] = face_w ? face_w[(size_t)F + m] : 0.0;
+    }
+    const double nrm[2] = {M.normal[m], M.normal[(size_t)F + m]};
+    double L[4], R[4], f[4];
+    ok = states64(A, C, dt_half, boost, linear, P.gizmo != 0, L, R) && ok;
+    int status = 0;
+    if (SOLVER == PHD_EXACT) {
+        if (ok) {
+            bool failed = false;
+            exact_flux<double, 2>(L, R, nrm, A.w, C.g, P.exact_max_iter, f, &failed);
+            if (failed) status = PHD_STATUS_RIEMANN_NONCONVERGED;
+        }
+    } else {
+        ok = hll64<SOLVER == PHD_HLLC>(L, R, nrm, A.w, C, boost, f) && ok;
+    }
+    if (ok) {
+        if (w) {
+            face_w[m] = A.w[0];
+            face_w[(size_t)F + m] = A.w[1];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) flux[(size_t)q * F + m] = f[q];
+    } else {
+        status = face_flux_plain(&M, &P, prim, grad, w, face_w, dt_half, m, i, j, flux);
+    }
+    set_status(clk, status);
 }
 
 // ---- conserved update -----------------------------------------------------------
@@ -789,19 +885,11 @@ __global__ void __launch_bounds__(BLOCK) k_face_vel(phd_mesh M, const double *__
     const int n = M.n_cells, F = M.n_faces;
     const int i = M.pair_i[m], j = M.pair_j[m];
     if (i < 0 || i >= n || j < 0 || j >= n) return;
-    double factor = 0.0, denom = 0.0;
-#pragma unroll
-    for (int k = 0; k < DIM; k++) {
-        const double xi = M.x[(size_t)k * n + i], xj = M.x[(size_t)k * n + j];
-        factor = factor + ((w[(size_t)k * n + i] - w[(size_t)k * n + j]) * (M.com[(size_t)k * F + m] - (0.5 * (xi + xj))));
-        denom = denom + t_sq(xj - xi);
-    }
-    factor = factor / denom;
-#pragma unroll
-    for (int k = 0; k < DIM; k++) {
-        const double xi = M.x[(size_t)k * n + i], xj = M.x[(size_t)k * n + j];
-        face_w[(size_t)k * F + m] = (0.5 * (w[(size_t)k * n + i] + w[(size_t)k * n + j])) + (factor * (xj - xi));
-    }
+    const double wi[2] = {w[i], w[(size_t)n + i]}, wj[2] = {w[j], w[(size_t)n + j]};
+    double fw[2];
+    face_velocity_plain(M, m, i, j, wi, wj, fw);
+    face_w[m] = fw[0];
+    face_w[(size_t)F + m] = fw[1];
 }
 
 inline int blk_of(int n) { return block_for(n, BLOCK); }
@@ -814,6 +902,20 @@ inline void launch_gradients(const phd_mesh &M, const double *prim, int limiter,
     const int grid = (M.n_cells + NC - 1) / NC;
     if (tape.f64) launch_pdl(k_gradients<NC, true>, grid, 4 * NC, stream, M, prim, (int)limiter, grad, clk, tape);
     else launch_pdl(k_gradients<NC, false>, grid, 4 * NC, stream, M, prim, (int)limiter, grad, clk, tape);
+}
+
+// Face fluxes; w: the generator velocities of a moving step, from which face_w is formed,
+// or null (face_w as given).
+inline void launch_face_flux(const phd_mesh &M, const phd_params &P, const double *prim, const double *grad,
+                             const double *w, double *face_w, double *flux, phd_clock *clk, cudaStream_t stream) {
+    const int block = block_for(M.n_faces, 128), grid = grid_for_block(M.n_faces, block);
+    const Gas64 C = gas64(P.gamma);
+    if (P.solver == PHD_HLL)
+        launch_pdl(k_face_flux<PHD_HLL>, grid, block, stream, M, P, C, prim, grad, w, face_w, flux, clk);
+    else if (P.solver == PHD_HLLC)
+        launch_pdl(k_face_flux<PHD_HLLC>, grid, block, stream, M, P, C, prim, grad, w, face_w, flux, clk);
+    else
+        launch_pdl(k_face_flux<PHD_EXACT>, grid, block, stream, M, P, C, prim, grad, w, face_w, flux, clk);
 }
 
 inline int launch_status() {
@@ -960,17 +1062,13 @@ static int step_f64(const phd_mesh *mesh, const phd_params *par, int32_t moving,
     const bool linear = par->reconstruction == PHD_LINEAR;
     if (linear && !grad) return PHD_ERR_ARG;
     if (moving && (!w || !face_w)) return PHD_ERR_ARG;
-    const int gc = grid_of(mesh->n_cells), gf = grid_of(mesh->n_faces);
-    const int bc = blk_of(mesh->n_cells), bf = blk_of(mesh->n_faces);
+    const int gc = grid_of(mesh->n_cells), bc = blk_of(mesh->n_cells);
     if (marks) cudaEventRecord(marks[0], stream);
-    if (moving) {
-        k_gen_vel<2><<<gc, bc, 0, stream>>>(*mesh, prim, par->gamma, par->eta, par->regularize, w);
-        if (mesh->n_faces) k_face_vel<2><<<gf, bf, 0, stream>>>(*mesh, w, face_w);
-    }
+    if (moving) k_gen_vel<2><<<gc, bc, 0, stream>>>(*mesh, prim, par->gamma, par->eta, par->regularize, w);
     if (linear) launch_gradients(*mesh, prim, par->limiter, grad, clk, tape, stream);
     if (marks) cudaEventRecord(marks[1], stream);
     if (mesh->n_faces)
-        k_face_flux<2><<<gf, bf, 0, stream>>>(*mesh, *par, prim, grad, face_w, flux, clk);
+        launch_face_flux(*mesh, *par, prim, grad, moving ? w : nullptr, face_w, flux, clk, stream);
     if (marks) cudaEventRecord(marks[2], stream);
     k_update_step<2><<<gc, bc, 0, stream>>>(*mesh, *par, flux, cons, cons_next, prim, clk);
     if (marks) cudaEventRecord(marks[3], stream);
