@@ -3,20 +3,20 @@
 // Forward step (real-cell conserved totals U -> U'):
 //   ghost refresh -> primitives -> limited gradients -> face states (spatial +
 //   GIZMO + MUSCL-Hancock half step) -> HLL/HLLC flux + deboost -> segmented update.
-// Reverse, five deterministic kernels (no atomics; every sum is a per-thread loop):
+// Reverse, three deterministic kernels (no atomics; every sum is a per-thread loop):
 //   k_adj_face     per face: flux adjoint dt*A*(lam'_j - lam'_i) through Riemann,
 //                  temporal and spatial stages -> 24 per-face adjoint values
-//   k_adj_gather   per cell: sum its faces' contributions -> lam_prim, lam_grad (own row)
-//   k_adj_grad     per real cell: fold ghost rows into lam_grad, reverse the limited
-//                  gradient -> per-entry neighbour adjoints and the cell's own adjoint
-//   k_adj_gather2  per cell: own + partner-entry contributions -> lam_prim
-//   k_adj_final    per real cell: fold ghost rows, reverse the primitive recovery,
-//                  lam = lam' + J^T lam_prim
+//   k_adj_cell     per cell: sum its faces' contributions; a real cell with its ghost rows
+//                  folded in, through the reverse of the limited gradient -> per-entry
+//                  neighbour adjoints and the cell's own adjoint
+//   k_adj_final    per real cell: own and ghost rows' sums and the neighbours' parts through
+//                  the reverse of the primitive recovery, lam = lam' + J^T lam_prim
 
 #include "phd_common.cuh"
 #include "phd_physics.cuh"
 #include "phd_adjoint.cuh"
 #include "phd_ref.cuh"
+#include "phd_adjface64.cuh"
 
 namespace phd {
 
@@ -104,130 +104,244 @@ __device__ __forceinline__ void spatial_rev_f64(const SpatialTape &t, const doub
     }
 }
 
-// EXACT: the exact solver's reverse (exact_flux_adj); otherwise HLL / HLLC -- separate
-// instantiations, so the HLL-family kernel carries none of the exact solver's registers.
+// One face on the plain path: 24 values to out.  EXACT: the exact solver's reverse
+// (exact_flux_adj); otherwise HLL / HLLC.
 template <bool EXACT>
-__global__ void __launch_bounds__(BA) k_adj_face(phd_mesh M, phd_params P, double dt, const double *__restrict__ prim,
-                                                 const double *__restrict__ grad, const double *__restrict__ face_w,
-                                                 const double *__restrict__ lam_next, double *__restrict__ out) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M.n_faces) return;
+__device__ __forceinline__ void adj_face_body(const phd_mesh &M, const phd_params &P, double dt, const double *prim,
+                                              const double *grad, const double *face_w, const double *lam_next, int m,
+                                              int i, int j, double *out) {
     const int n = M.n_cells, F = M.n_faces;
-    const int i = M.pair_i[m], j = M.pair_j[m];
     double res[FACE_ADJ];
     for (int q = 0; q < FACE_ADJ; q++) res[q] = 0.0;
-    if (i >= 0 && i < n && j >= 0 && j < n) {
-        const bool boost = (P.boost != 0);
-        const bool linear = P.reconstruction == PHD_LINEAR;
-        double pi[4], pj[4], gi[8], gj[8], w[2], nrm[2];
-        for (int f = 0; f < 4; f++) { pi[f] = prim[(size_t)f * n + i]; pj[f] = prim[(size_t)f * n + j]; }
-        for (int r = 0; r < 8; r++) {
-            gi[r] = linear ? grad[(size_t)r * n + i] : 0.0;
-            gj[r] = linear ? grad[(size_t)r * n + j] : 0.0;
-        }
-        for (int k = 0; k < 2; k++) {
-            w[k] = face_w ? face_w[(size_t)k * F + m] : 0.0;
-            nrm[k] = M.normal[(size_t)k * F + m];
-        }
-        // flux adjoint from the update U_i -= dt a F, U_j += dt a F (j real)
-        const double da = dt * M.area[m];
-        const bool jr = M.tag[j] == PHD_REAL_TAG;
-        double aF[4];
-        for (int q = 0; q < 4; q++)
-            aF[q] = da * ((jr ? lam_next[(size_t)q * n + j] : 0.0) - lam_next[(size_t)q * n + i]);
-        // forward states (the spatial stage once, its tape kept for the reverse)
-        double Ls[4], Rs[4], L[4], R[4];
-        SpatialTape tape;
-        if (linear) {
-            spatial_fwd_f64(M, m, i, j, pi, pj, gi, gj, w, boost, P.gizmo != 0, tape, Ls, Rs);
-            for (int f = 0; f < 4; f++) { L[f] = Ls[f]; R[f] = Rs[f]; }
-            temporal<double, 2>(L, R, pi, pj, gi, gj, w, P.gamma, 0.5 * dt, boost);
-        } else {
-            for (int f = 0; f < 4; f++) { L[f] = pi[f]; R[f] = pj[f]; }
-            if (boost) for (int k = 0; k < 2; k++) { L[1 + k] -= w[k]; R[1 + k] -= w[k]; }
-        }
-        double aL[4] = {0, 0, 0, 0}, aR[4] = {0, 0, 0, 0};
-        if (EXACT) exact_flux_adj(L, R, nrm, w, P.gamma, P.exact_max_iter, aF, aL, aR);
-        else hll_family_adj<double>(P.solver == PHD_HLLC, L, R, nrm, w, P.gamma, boost, aF, aL, aR);
-        double *api = res, *apj = res + 4, *agi = res + 8, *agj = res + 16;
-        if (linear) {
-            double aLs[4] = {0, 0, 0, 0}, aRs[4] = {0, 0, 0, 0};
-            temporal_adj<double>(Ls, Rs, pi, pj, gi, gj, w, P.gamma, 0.5 * dt, boost, aL, aR, aLs, aRs, api, apj,
-                                 agi, agj);
-            spatial_rev_f64(tape, pi, pj, P.gizmo != 0, aLs, aRs, api, apj, agi, agj);
-        } else {
-            for (int f = 0; f < 4; f++) { api[f] += aL[f]; apj[f] += aR[f]; }
-        }
+    const bool boost = (P.boost != 0);
+    const bool linear = P.reconstruction == PHD_LINEAR;
+    double pi[4], pj[4], gi[8], gj[8], w[2], nrm[2];
+    for (int f = 0; f < 4; f++) { pi[f] = prim[(size_t)f * n + i]; pj[f] = prim[(size_t)f * n + j]; }
+    for (int r = 0; r < 8; r++) {
+        gi[r] = linear ? grad[(size_t)r * n + i] : 0.0;
+        gj[r] = linear ? grad[(size_t)r * n + j] : 0.0;
+    }
+    for (int k = 0; k < 2; k++) {
+        w[k] = face_w ? face_w[(size_t)k * F + m] : 0.0;
+        nrm[k] = M.normal[(size_t)k * F + m];
+    }
+    // flux adjoint from the update U_i -= dt a F, U_j += dt a F (j real)
+    const double da = dt * M.area[m];
+    const bool jr = M.tag[j] == PHD_REAL_TAG;
+    double aF[4];
+    for (int q = 0; q < 4; q++)
+        aF[q] = da * ((jr ? lam_next[(size_t)q * n + j] : 0.0) - lam_next[(size_t)q * n + i]);
+    // forward states (the spatial stage once, its tape kept for the reverse)
+    double Ls[4], Rs[4], L[4], R[4];
+    SpatialTape tape;
+    if (linear) {
+        spatial_fwd_f64(M, m, i, j, pi, pj, gi, gj, w, boost, P.gizmo != 0, tape, Ls, Rs);
+        for (int f = 0; f < 4; f++) { L[f] = Ls[f]; R[f] = Rs[f]; }
+        temporal<double, 2>(L, R, pi, pj, gi, gj, w, P.gamma, 0.5 * dt, boost);
+    } else {
+        for (int f = 0; f < 4; f++) { L[f] = pi[f]; R[f] = pj[f]; }
+        if (boost) for (int k = 0; k < 2; k++) { L[1 + k] -= w[k]; R[1 + k] -= w[k]; }
+    }
+    double aL[4] = {0, 0, 0, 0}, aR[4] = {0, 0, 0, 0};
+    if (EXACT) exact_flux_adj(L, R, nrm, w, P.gamma, P.exact_max_iter, aF, aL, aR);
+    else hll_family_adj<double>(P.solver == PHD_HLLC, L, R, nrm, w, P.gamma, boost, aF, aL, aR);
+    double *api = res, *apj = res + 4, *agi = res + 8, *agj = res + 16;
+    if (linear) {
+        double aLs[4] = {0, 0, 0, 0}, aRs[4] = {0, 0, 0, 0};
+        temporal_adj<double>(Ls, Rs, pi, pj, gi, gj, w, P.gamma, 0.5 * dt, boost, aL, aR, aLs, aRs, api, apj,
+                             agi, agj);
+        spatial_rev_f64(tape, pi, pj, P.gizmo != 0, aLs, aRs, api, apj, agi, agj);
+    } else {
+        for (int f = 0; f < 4; f++) { api[f] += aL[f]; apj[f] += aR[f]; }
     }
     for (int q = 0; q < FACE_ADJ; q++) out[(size_t)q * F + m] = res[q];
 }
 
-// per cell: sum of its faces' contributions (own row, ghosts included)
-__global__ void __launch_bounds__(BA) k_adj_gather(phd_mesh M, const double *__restrict__ face_adj,
-                                                   double *__restrict__ cell_adj /* [12][n] */) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= M.n_cells) return;
+__device__ __noinline__ void adj_face_plain(const phd_mesh *M, const phd_params *P, double dt, const double *prim,
+                                            const double *grad, const double *face_w, const double *lam_next, int m,
+                                            int i, int j, double *out) {
+    adj_face_body<false>(*M, *P, dt, prim, grad, face_w, lam_next, m, i, j, out);
+}
+
+// The exact solver's faces (220 registers).
+__global__ void __launch_bounds__(BA) k_adj_face_exact(phd_mesh M, phd_params P, double dt, const double *__restrict__ prim,
+                                                       const double *__restrict__ grad,
+                                                       const double *__restrict__ face_w,
+                                                       const double *__restrict__ lam_next, double *__restrict__ out) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= M.n_faces) return;
+    const int i = M.pair_i[m], j = M.pair_j[m];
+    if (i < 0 || i >= M.n_cells || j < 0 || j >= M.n_cells) {
+        for (int q = 0; q < FACE_ADJ; q++) out[(size_t)q * M.n_faces + m] = 0.0;
+        return;
+    }
+    adj_face_body<true>(M, P, dt, prim, grad, face_w, lam_next, m, i, j, out);
+}
+
+// HLL / HLLC: the lean reverse (phd_adjface64.cuh), the plain one for the faces it declines.
+// Bound by the FP64 pipe; held to 168 registers for 12 warps an SM (the pipe waits on 8 at 255:
+// 14.0 against 15.1 ms for 40 steps forward and backward at 128 x 128).  Measured there (50,000
+// faces, HLLC, cold caches): 317 -> 102 us at 255 registers, 2157 -> 657 FP64 instructions per
+// warp.
+template <bool HLLC>
+__global__ void __launch_bounds__(128, 3) k_adj_face(const __grid_constant__ phd_mesh M, const __grid_constant__ phd_params P,
+                                                  const __grid_constant__ Gas64 C, double dt,
+                                                  const double *__restrict__ prim, const double *__restrict__ grad,
+                                                  const double *__restrict__ face_w,
+                                                  const double *__restrict__ lam_next, double *__restrict__ out) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= M.n_faces) return;
     const int n = M.n_cells, F = M.n_faces;
-    double s[12];
+    const int i = M.pair_i[m], j = M.pair_j[m];
+    if (i < 0 || i >= n || j < 0 || j >= n) {
+        for (int q = 0; q < FACE_ADJ; q++) out[(size_t)q * F + m] = 0.0;
+        return;
+    }
+    const bool boost = P.boost != 0, linear = P.reconstruction == PHD_LINEAR, gizmo = P.gizmo != 0;
+    Face64 A;
+#pragma unroll
+    for (int f = 0; f < 4; f++) { A.pi[f] = prim[(size_t)f * n + i]; A.pj[f] = prim[(size_t)f * n + j]; }
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        A.gi[r] = linear ? grad[(size_t)r * n + i] : 0.0;
+        A.gj[r] = linear ? grad[(size_t)r * n + j] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        A.w[k] = face_w ? face_w[(size_t)k * F + m] : 0.0;
+        A.xi[k] = M.x[(size_t)k * n + i];
+        A.xj[k] = M.x[(size_t)k * n + j];
+        A.ci[k] = M.dcom[(size_t)k * n + i];
+        A.cj[k] = M.dcom[(size_t)k * n + j];
+        A.com[k] = M.com[(size_t)k * F + m];
+    }
+    const double nrm[2] = {M.normal[m], M.normal[(size_t)F + m]};
+    // flux adjoint from the update U_i -= dt a F, U_j += dt a F (j real)
+    const double da = dt * M.area[m];
+    const bool jr = M.tag[j] == PHD_REAL_TAG;
+    double aF[4], sl[4], sr[4], L[4], R[4], aL[4] = {0., 0., 0., 0.}, aR[4] = {0., 0., 0., 0.};
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        aF[q] = da * ((jr ? lam_next[(size_t)q * n + j] : 0.0) - lam_next[(size_t)q * n + i]);
+    StateDecisions D;
+    bool ok;
+    if (linear) {
+        ok = states64_decide(A, C, 0.5 * dt, boost, gizmo, sl, sr, L, R, D);
+    } else {
+        ok = states64(A, C, 0.5 * dt, boost, false, false, L, R);
+    }
+    ok = ok && hll64_adj<HLLC>(L, R, nrm, A.w, C, boost, aF, aL, aR);
+    if (ok && !linear) {
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            out[(size_t)f * F + m] = aL[f];
+            out[(size_t)(4 + f) * F + m] = aR[f];
+        }
+#pragma unroll
+        for (int r = 8; r < 24; r++) out[(size_t)r * F + m] = 0.;
+    } else if (ok) {
+        double asl[4], aol[4], asr[4], aor[4], agl[8], agr[8], rl, pl, rr, pr;
+        side64_rev(aL, D.half_l, D.spat_l, gizmo, false, D, A.pi, A.gi, sl, sr, C.g, 0.5 * dt, asl, aol, agl, rl, pl, ok);
+        side64_rev(aR, D.half_r, D.spat_r, gizmo, true, D, A.pj, A.gj, sr, sl, C.g, 0.5 * dt, asr, aor, agr, rr, pr, ok);
+        if (ok) {
+#pragma unroll
+            for (int f = 0; f < 4; f++) {
+                const double hi = f == 0 ? rl : (f == 3 ? pl : 0.), hj = f == 0 ? rr : (f == 3 ? pr : 0.);
+                out[(size_t)f * F + m] = (asl[f] + hi) + aor[f];
+                out[(size_t)(4 + f) * F + m] = (asr[f] + hj) + aol[f];
+            }
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                out[(size_t)(8 + r) * F + m] = agl[r];
+                out[(size_t)(16 + r) * F + m] = agr[r];
+            }
+        }
+    }
+    if (!ok) adj_face_plain(&M, &P, dt, prim, grad, face_w, lam_next, m, i, j, out);
+}
+
+// Sum of row x's face contributions (12 values: primitives, gradients), in list order.
+__device__ __forceinline__ void gather_row(const phd_mesh &M, const double *__restrict__ face_adj, int x, double *s) {
+    const int F = M.n_faces;
+#pragma unroll
     for (int q = 0; q < 12; q++) s[q] = 0.0;
     for (int e = M.nbr_ptr[x]; e < M.nbr_ptr[x + 1]; e++) {
         const int f = M.nbr_idx[e];
         if (f < 0 || f >= F) continue;
         const bool as_i = M.pair_i[f] == x;
-        const int pbase = as_i ? 0 : 4, gbase = as_i ? 8 : 16;
-        for (int q = 0; q < 4; q++) s[q] += face_adj[(size_t)(pbase + q) * F + f];
-        for (int q = 0; q < 8; q++) s[4 + q] += face_adj[(size_t)(gbase + q) * F + f];
+        const size_t pb = as_i ? 0 : 4, gb = as_i ? 8 : 16;
+#pragma unroll
+        for (int q = 0; q < 4; q++) s[q] += face_adj[(pb + q) * F + f];
+#pragma unroll
+        for (int q = 0; q < 8; q++) s[4 + q] += face_adj[(gb + q) * F + f];
     }
-    for (int q = 0; q < 12; q++) cell_adj[(size_t)q * n + x] = s[q];
 }
 
-// per real cell: reverse of the limited gradient (cell_gradient_f64).
+// Per real cell: its rows' face contributions (own and ghosts', with the reflective flips)
+// and the reverse of the limited gradient (cell_gradient_f64): the primitives' part to
+// prim_part, the neighbours' to entry_adj, the own one added to prim_part.  Ghost rows' entries
+// get zeros (their gradient is their image's).  LINEAR: false for constant reconstruction,
+// which has no gradients.
 // TAPED: the forward selections (unlimited estimate, limiter values, active entries,
 // neighbour extrema) come from the limiter record of a taped forward step instead of
 // being recomputed.
-template <bool TAPED>
-__global__ void __launch_bounds__(BA) k_adj_grad(phd_mesh M, phd_adj_index A, int limiter,
-                                                 const double *__restrict__ prim, const double *__restrict__ cell_adj,
-                                                 double *__restrict__ entry_adj /* [4][2F] */,
-                                                 double *__restrict__ self_adj /* [4][n] */,
-                                                 const double *__restrict__ tape_f64,
-                                                 const int32_t *__restrict__ tape_i32) {
+// One kernel where a gather per cell, two clears and this reverse were four launches; the
+// reverse's own arithmetic is fused multiply-adds on a reciprocal per entry (phd_fp64.cuh),
+// 38 FP64 instructions an entry instead of 80.
+template <bool LINEAR, bool TAPED>
+__global__ void __launch_bounds__(128) k_adj_cell(const __grid_constant__ phd_mesh M, phd_adj_index A, int limiter,
+                                                  const double *__restrict__ prim, const double *__restrict__ face_adj,
+                                                  double *__restrict__ entry_adj /* [4][2F] */,
+                                                  double *__restrict__ prim_part /* [4][n] */,
+                                                  const double *__restrict__ tape_f64,
+                                                  const int32_t *__restrict__ tape_i32) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= M.n_cells || M.tag[c] != PHD_REAL_TAG) return;
+    if (c >= M.n_cells) return;
     const int n = M.n_cells, F = M.n_faces;
-    const int E2 = 2 * F;
+    const size_t E2 = 2 * (size_t)F;
+    const int m0 = M.nbr_ptr[c], m1 = M.nbr_ptr[c + 1];
+    double own[12];
+    if (M.tag[c] != PHD_REAL_TAG) {
+        gather_row(M, face_adj, c, own);             // the primitives' part, folded by k_adj_final
+#pragma unroll
+        for (int f = 0; f < 4; f++) prim_part[(size_t)f * n + c] = own[f];
+        if (LINEAR)
+            for (int e = m0; e < m1; e++)
+#pragma unroll
+                for (int f = 0; f < 4; f++) entry_adj[f * E2 + e] = 0.0;
+        return;
+    }
+    gather_row(M, face_adj, c, own);
+    if (!LINEAR) {
+#pragma unroll
+        for (int f = 0; f < 4; f++) prim_part[(size_t)f * n + c] = own[f];
+        return;
+    }
     // lam_grad of this cell = own row + its ghost rows (reflective diagonal flip)
-    double ag[8];
-    for (int q = 0; q < 8; q++) ag[q] = cell_adj[(size_t)(4 + q) * n + c];
+    double *ag = own + 4;
     for (int t = A.ghost_ptr[c]; t < A.ghost_ptr[c + 1]; t++) {
         const int g = A.ghost_idx[t];
         const int fl = M.flip ? M.flip[g] : 0;
-        for (int q = 0; q < 8; q++) {
-            double v = cell_adj[(size_t)(4 + q) * n + g];
-            if ((q == 2 && (fl & 1)) || (q == 5 && (fl & 2))) v = -v;
-            ag[q] += v;
-        }
+        double row[12];
+        gather_row(M, face_adj, g, row);
+        if (fl & 1) row[6] = -row[6];
+        if (fl & 2) row[9] = -row[9];
+#pragma unroll
+        for (int q = 0; q < 8; q++) ag[q] += row[4 + q];
     }
-    // forward recompute (cell_gradient_f64 with selections)
-    double xi[2], cx[2], pc[4], df[8], phi_max[4], phi_min[4];
+    double xi[2], cx[2], pc[4], df[8], alpha[4] = {1.0, 1.0, 1.0, 1.0};
     int arg_max[4], arg_min[4];
+    int act[4] = {-1, -1, -1, -1};     // entry whose psi is the active limit
+    int act_f0 = -1;                   // TESS: field of the active psi
     for (int k = 0; k < 2; k++) {
         xi[k] = M.x[(size_t)k * n + c];
         cx[k] = xi[k] + M.dcom[(size_t)k * n + c];
     }
     const double vol = M.vol[c];
-    for (int f = 0; f < 4; f++) {
-        pc[f] = prim[(size_t)f * n + c];
-        phi_max[f] = phi_min[f] = pc[f];
-        arg_max[f] = arg_min[f] = -1;
-        df[2 * f] = df[2 * f + 1] = 0.0;
-    }
-    const int m0 = M.nbr_ptr[c], m1 = M.nbr_ptr[c + 1];
-    double alpha[4] = {1.0, 1.0, 1.0, 1.0};
-    int act[4] = {-1, -1, -1, -1};     // entry whose psi is the active limit
-    int act_f0 = -1;                   // TESS: field of the active psi
     if (TAPED) {
+#pragma unroll
         for (int r = 0; r < 8; r++) df[r] = tape_f64[(size_t)r * n + c];
+#pragma unroll
         for (int f = 0; f < 4; f++) {
             alpha[f] = tape_f64[(size_t)(8 + f) * n + c];
             act[f] = tape_i32[(size_t)f * n + c];
@@ -235,178 +349,187 @@ __global__ void __launch_bounds__(BA) k_adj_grad(phd_mesh M, phd_adj_index A, in
             arg_min[f] = tape_i32[(size_t)(8 + f) * n + c];
         }
         act_f0 = tape_i32[(size_t)12 * n + c];
-    }
-    for (int e = m0; e < (TAPED ? m0 : m1); e++) {
-        const int fid = M.nbr_idx[e];
-        const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
-        const double area = M.area[fid];
-        double cfx[2], dr[2], r = 0.0;
-        for (int k = 0; k < 2; k++) {
-            const double xj = M.x[(size_t)k * n + j];
-            cfx[k] = M.com[(size_t)k * F + fid] - 0.5 * (xi[k] + xj);
-            dr[k] = xi[k] - xj;
-            r = r + t_sq(dr[k]);
-        }
-        r = sqrt(r);
+    } else {
+        // forward recompute (cell_gradient_f64 with selections)
+        double phi_max[4], phi_min[4];
         for (int f = 0; f < 4; f++) {
-            const double pj = prim[(size_t)f * n + j];
-            if (pj > phi_max[f]) { phi_max[f] = pj; arg_max[f] = e; }
-            if (pj < phi_min[f]) { phi_min[f] = pj; arg_min[f] = e; }
-            const double d_dif = pj - pc[f], d_sum = pj + pc[f];
-            for (int k = 0; k < 2; k++)
-                df[2 * f + k] = df[2 * f + k] + (area * ((d_dif * cfx[k]) - ((0.5 * d_sum) * dr[k]))) / (r * vol);
+            pc[f] = prim[(size_t)f * n + c];
+            phi_max[f] = phi_min[f] = pc[f];
+            arg_max[f] = arg_min[f] = -1;
+            df[2 * f] = df[2 * f + 1] = 0.0;
         }
-    }
-    for (int e = m0; e < (TAPED ? m0 : m1); e++) {
-        const int fid = M.nbr_idx[e];
-        const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
-        double sep[2];
-        for (int k = 0; k < 2; k++) sep[k] = M.com[(size_t)k * F + fid] - cx[k];
-        for (int f = 0; f < 4; f++) {
-            double dphi = 0.0, psi;
-            for (int k = 0; k < 2; k++) dphi = dphi + df[2 * f + k] * sep[k];
-            if (limiter == PHD_LIMITER_AREPO) {
-                if (dphi > 0) psi = (phi_max[f] - pc[f]) / dphi;
-                else if (dphi < 0) psi = (phi_min[f] - pc[f]) / dphi;
-                else psi = 1.0;
-                const double cand = fmax(psi, 0.);
-                if (cand < alpha[f]) { alpha[f] = cand; act[f] = (psi > 0.0 && dphi != 0.0) ? e : -2; }
-            } else {
-                if (dphi > 0.0 || dphi < 0.0) {
-                    const double t = (prim[(size_t)f * n + j] - pc[f]) / dphi;
-                    psi = (0. > t) ? 0. : t;
-                } else psi = 1.0;
-                const double cand = fmax(psi, 0.);
-                if (cand < alpha[0]) { alpha[0] = cand; act[0] = (psi > 0.0 && dphi != 0.0) ? e : -2; act_f0 = f; }
+        for (int e = m0; e < m1; e++) {
+            const int fid = M.nbr_idx[e];
+            const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
+            const double area = M.area[fid];
+            double cfx[2], dr[2], r = 0.0;
+            for (int k = 0; k < 2; k++) {
+                const double xj = M.x[(size_t)k * n + j];
+                cfx[k] = M.com[(size_t)k * F + fid] - 0.5 * (xi[k] + xj);
+                dr[k] = xi[k] - xj;
+                r = r + t_sq(dr[k]);
+            }
+            r = sqrt(r);
+            for (int f = 0; f < 4; f++) {
+                const double pj = prim[(size_t)f * n + j];
+                if (pj > phi_max[f]) { phi_max[f] = pj; arg_max[f] = e; }
+                if (pj < phi_min[f]) { phi_min[f] = pj; arg_min[f] = e; }
+                const double d_dif = pj - pc[f], d_sum = pj + pc[f];
+                for (int k = 0; k < 2; k++)
+                    df[2 * f + k] = df[2 * f + k] + (area * ((d_dif * cfx[k]) - ((0.5 * d_sum) * dr[k]))) / (r * vol);
+            }
+        }
+        for (int e = m0; e < m1; e++) {
+            const int fid = M.nbr_idx[e];
+            const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
+            double sep[2];
+            for (int k = 0; k < 2; k++) sep[k] = M.com[(size_t)k * F + fid] - cx[k];
+            for (int f = 0; f < 4; f++) {
+                double dphi = 0.0, psi;
+                for (int k = 0; k < 2; k++) dphi = dphi + df[2 * f + k] * sep[k];
+                if (limiter == PHD_LIMITER_AREPO) {
+                    if (dphi > 0) psi = (phi_max[f] - pc[f]) / dphi;
+                    else if (dphi < 0) psi = (phi_min[f] - pc[f]) / dphi;
+                    else psi = 1.0;
+                    const double cand = fmax(psi, 0.);
+                    if (cand < alpha[f]) { alpha[f] = cand; act[f] = (psi > 0.0 && dphi != 0.0) ? e : -2; }
+                } else {
+                    if (dphi > 0.0 || dphi < 0.0) {
+                        const double t = (prim[(size_t)f * n + j] - pc[f]) / dphi;
+                        psi = (0. > t) ? 0. : t;
+                    } else psi = 1.0;
+                    const double cand = fmax(psi, 0.);
+                    if (cand < alpha[0]) { alpha[0] = cand; act[0] = (psi > 0.0 && dphi != 0.0) ? e : -2; act_f0 = f; }
+                }
             }
         }
     }
     // reverse: grad = alpha * df
     double adf[8], aself[4] = {0, 0, 0, 0}, aalpha[4];
+#pragma unroll
     for (int f = 0; f < 4; f++) {
-        aalpha[f] = 0.0;
-        for (int k = 0; k < 2; k++) {
-            adf[2 * f + k] = alpha[f] * ag[2 * f + k];
-            aalpha[f] += df[2 * f + k] * ag[2 * f + k];
-        }
+        aalpha[f] = fma(df[2 * f], ag[2 * f], df[2 * f + 1] * ag[2 * f + 1]);
+        adf[2 * f] = alpha[f] * ag[2 * f];
+        adf[2 * f + 1] = alpha[f] * ag[2 * f + 1];
     }
     // limiter: active psi -> (extreme value, own value, df)
-    double aext[4] = {0, 0, 0, 0};       // AREPO: adjoint of phi_max / phi_min of field f
-    int ext_arg[4] = {-1, -1, -1, -1};
-    int tess_e = -1, tess_f = -1;
-    double tess_aj = 0.0;
+    double aext[4] = {0, 0, 0, 0};       // adjoint of the active entry's phi_max / phi_min (TESS: neighbour)
+    int ext[4] = {-1, -1, -1, -1};       // and the entry it belongs to (-1: the cell itself)
+    const bool tess = limiter == PHD_LIMITER_TESS;
+#pragma unroll
     for (int f = 0; f < 4; f++) {
         const int e = act[f];
-        if (e < 0) continue;
-        if (limiter == PHD_LIMITER_TESS && f != 0) continue;
-        const int ff = (limiter == PHD_LIMITER_TESS) ? act_f0 : f;
-        const int fid = M.nbr_idx[e];
-        double sep[2];
-        for (int k = 0; k < 2; k++) sep[k] = M.com[(size_t)k * F + fid] - cx[k];
-        double dphi = 0.0;
-        for (int k = 0; k < 2; k++) dphi = dphi + df[2 * ff + k] * sep[k];
-        const double apsi = aalpha[f];
-        const double psi = alpha[f];
-        const double adphi = -apsi * psi / dphi;
-        for (int k = 0; k < 2; k++) adf[2 * ff + k] += adphi * sep[k];
-        aself[ff] -= apsi / dphi;
-        if (limiter == PHD_LIMITER_AREPO) {
-            aext[ff] += apsi / dphi;
-            ext_arg[ff] = dphi > 0 ? arg_max[ff] : arg_min[ff];
-        } else {
-            tess_e = e;
-            tess_f = ff;
-            tess_aj = apsi / dphi;
+        if (e < 0 || (tess && f != 0)) continue;
+        const int ff = tess ? act_f0 : f, fid = M.nbr_idx[e];
+        const double s0 = M.com[fid] - cx[0], s1 = M.com[(size_t)F + fid] - cx[1];
+        double d0 = df[2 * f], d1 = df[2 * f + 1];
+        if (tess) {
+#pragma unroll
+            for (int g = 0; g < 4; g++) { d0 = g == ff ? df[2 * g] : d0; d1 = g == ff ? df[2 * g + 1] : d1; }
         }
+        const double dphi = d0 * s0 + d1 * s1;
+        bool ok = true;
+        double y = f64_rcp(dphi, ok);
+        if (!ok) y = 1.0 / dphi;
+        const double ap = aalpha[f] * y, ad = -ap * alpha[f];
+        const int arg = tess ? e : (f64_pos(dphi) ? arg_max[f] : arg_min[f]);
+#pragma unroll
+        for (int g = 0; g < 4; g++)
+            if (g == ff) {
+                adf[2 * g] = fma(ad, s0, adf[2 * g]);
+                adf[2 * g + 1] = fma(ad, s1, adf[2 * g + 1]);
+                aself[g] -= ap;
+                if (arg >= 0) {
+                    aext[g] = ap;
+                    ext[g] = arg;
+                } else {
+                    aself[g] += ap;
+                }
+            }
     }
-    for (int f = 0; f < 4; f++)
-        if (limiter == PHD_LIMITER_AREPO && aext[f] != 0.0 && ext_arg[f] < 0) aself[f] += aext[f];
     // df = sum_e area (d_dif cfx - d_sum dr / 2) / (r vol)
     for (int e = m0; e < m1; e++) {
         const int fid = M.nbr_idx[e];
         const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
         const double area = M.area[fid];
-        double cfx[2], dr[2], r = 0.0;
-        for (int k = 0; k < 2; k++) {
-            const double xj = M.x[(size_t)k * n + j];
-            cfx[k] = M.com[(size_t)k * F + fid] - 0.5 * (xi[k] + xj);
-            dr[k] = xi[k] - xj;
-            r = r + t_sq(dr[k]);
+        const double xj = M.x[j], yj = M.x[(size_t)n + j];
+        const double cfx = fma(-0.5, xi[0] + xj, M.com[fid]), cfy = fma(-0.5, xi[1] + yj, M.com[(size_t)F + fid]);
+        const double dx = xi[0] - xj, dy = xi[1] - yj;
+        bool ok = true;
+        double r2 = fma(dx, dx, dy * dy), r = f64_sqrt(r2, ok), y = f64_rcp(r * vol, ok);
+        if (!ok) {
+            r = sqrt(r2);
+            y = 1.0 / (r * vol);
         }
-        r = sqrt(r);
-        const double coef = area / (r * vol);
-        double aj[4];
+        const double coef = area * y;
+        const double jx = coef * fma(-0.5, dx, cfx), jy = coef * fma(-0.5, dy, cfy);      // d df / d phi_j
+        const double sx = -coef * fma(0.5, dx, cfx), sy = -coef * fma(0.5, dy, cfy);      // d df / d phi_c
+#pragma unroll
         for (int f = 0; f < 4; f++) {
-            double sj = 0.0, sc = 0.0;
-            for (int k = 0; k < 2; k++) {
-                sj += adf[2 * f + k] * (cfx[k] - 0.5 * dr[k]);
-                sc += adf[2 * f + k] * (-cfx[k] - 0.5 * dr[k]);
-            }
-            aj[f] = sj * coef;
-            aself[f] += sc * coef;
-            if (limiter == PHD_LIMITER_AREPO && ext_arg[f] == e) aj[f] += aext[f];
-            if (limiter == PHD_LIMITER_TESS && tess_e == e && tess_f == f) aj[f] += tess_aj;
+            double aj = fma(adf[2 * f], jx, adf[2 * f + 1] * jy);
+            aself[f] = fma(adf[2 * f], sx, fma(adf[2 * f + 1], sy, aself[f]));
+            if (ext[f] == e) aj += aext[f];
+            entry_adj[f * E2 + e] = aj;
         }
-        for (int f = 0; f < 4; f++) entry_adj[(size_t)f * E2 + e] = aj[f];
     }
-    for (int f = 0; f < 4; f++) self_adj[(size_t)f * n + c] = aself[f];
+#pragma unroll
+    for (int f = 0; f < 4; f++) prim_part[(size_t)f * n + c] = own[f] + aself[f];
 }
 
-// per cell: primitive adjoint = face part + own gradient part + neighbours' gradient parts
-__global__ void __launch_bounds__(BA) k_adj_gather2(phd_mesh M, phd_adj_index A, const double *__restrict__ cell_adj,
-                                                    const double *__restrict__ entry_adj,
-                                                    const double *__restrict__ self_adj,
-                                                    double *__restrict__ prim_adj /* [4][n] */) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= M.n_cells) return;
-    const int n = M.n_cells, E2 = 2 * M.n_faces;
-    const bool real = M.tag[x] == PHD_REAL_TAG;
-    double s[4];
-    for (int f = 0; f < 4; f++) s[f] = cell_adj[(size_t)f * n + x] + (real ? self_adj[(size_t)f * n + x] : 0.0);
-    for (int e = M.nbr_ptr[x]; e < M.nbr_ptr[x + 1]; e++) {
-        const int pe = A.partner[e];
-        if (pe < 0 || pe >= E2) continue;
-        for (int f = 0; f < 4; f++) s[f] += entry_adj[(size_t)f * E2 + pe];
-    }
-    for (int f = 0; f < 4; f++) prim_adj[(size_t)f * n + x] = s[f];
-}
-
-// per real cell: fold ghosts, reverse primitive recovery, add the identity of the update
-__global__ void __launch_bounds__(BA) k_adj_final(phd_mesh M, phd_adj_index A, double gamma,
-                                                  const double *__restrict__ cons, const double *__restrict__ prim_adj,
-                                                  const double *__restrict__ lam_next, double *__restrict__ lam) {
+// Per real cell: its rows' primitive adjoints (own and ghosts', flipped) with the neighbours'
+// gradient parts, through the primitive recovery, plus the identity of the update; ghost
+// rows of lam are zero.
+template <bool LINEAR>
+__global__ void __launch_bounds__(128) k_adj_final(const __grid_constant__ phd_mesh M, phd_adj_index A, double gamma,
+                                                   const double *__restrict__ cons, const double *__restrict__ prim_part,
+                                                   const double *__restrict__ entry_adj,
+                                                   const double *__restrict__ lam_next, double *__restrict__ lam) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= M.n_cells) return;
     const int n = M.n_cells;
+    const size_t E2 = 2 * (size_t)M.n_faces;
     if (M.tag[c] != PHD_REAL_TAG) {
         for (int q = 0; q < 4; q++) lam[(size_t)q * n + c] = 0.0;
         return;
     }
-    double ap[4];
-    for (int f = 0; f < 4; f++) ap[f] = prim_adj[(size_t)f * n + c];
-    for (int t = A.ghost_ptr[c]; t < A.ghost_ptr[c + 1]; t++) {
-        const int g = A.ghost_idx[t];
-        const int fl = M.flip ? M.flip[g] : 0;
-        for (int f = 0; f < 4; f++) {
-            double v = prim_adj[(size_t)f * n + g];
-            if ((f == 1 && (fl & 1)) || (f == 2 && (fl & 2))) v = -v;
-            ap[f] += v;
+    double ap[4] = {0., 0., 0., 0.};
+    const int t0 = A.ghost_ptr[c], t1 = A.ghost_ptr[c + 1];
+    for (int t = t0 - 1; t < t1; t++) {              // the cell itself, then its ghosts
+        const int x = t < t0 ? c : A.ghost_idx[t];
+        const int fl = (t >= t0 && M.flip) ? M.flip[x] : 0;
+        double s[4];
+#pragma unroll
+        for (int f = 0; f < 4; f++) s[f] = prim_part[(size_t)f * n + x];
+        if (LINEAR) {
+            for (int e = M.nbr_ptr[x]; e < M.nbr_ptr[x + 1]; e++) {
+                const int pe = A.partner[e];
+                if (pe < 0 || (size_t)pe >= E2) continue;
+#pragma unroll
+                for (int f = 0; f < 4; f++) s[f] += entry_adj[f * E2 + pe];
+            }
         }
+        if (fl & 1) s[1] = -s[1];
+        if (fl & 2) s[2] = -s[2];
+#pragma unroll
+        for (int f = 0; f < 4; f++) ap[f] += s[f];
     }
     const double m = cons[c], mx = cons[(size_t)n + c], my = cons[2 * (size_t)n + c];
     const double vol = M.vol[c];
-    const double rho = m / vol, vx = mx / m, vy = my / m;
-    const double g1 = gamma - 1.0;
+    bool ok = true;
+    double im = f64_rcp(m, ok), iv = f64_rcp(vol, ok);
+    if (!ok) {
+        im = 1.0 / m;
+        iv = 1.0 / vol;
+    }
+    const double rho = m * iv, vx = mx * im, vy = my * im;
+    const double g1 = gamma - 1.0, a3 = ap[3] * g1;
     // p = (E/V - rho v^2 / 2)(gamma - 1)
-    const double arho = ap[0] - ap[3] * 0.5 * (vx * vx + vy * vy) * g1;
-    const double avx = ap[1] - ap[3] * rho * vx * g1;
-    const double avy = ap[2] - ap[3] * rho * vy * g1;
-    const double aE = ap[3] * g1 / vol;
-    const double am = arho / vol - avx * vx / m - avy * vy / m;
-    lam[c] = lam_next[c] + am;
-    lam[(size_t)n + c] = lam_next[(size_t)n + c] + avx / m;
-    lam[2 * (size_t)n + c] = lam_next[2 * (size_t)n + c] + avy / m;
-    lam[3 * (size_t)n + c] = lam_next[3 * (size_t)n + c] + aE;
+    const double arho = fma(-0.5 * a3, fma(vx, vx, vy * vy), ap[0]);
+    const double ax = fma(-a3 * rho, vx, ap[1]) * im, ay = fma(-a3 * rho, vy, ap[2]) * im;
+    lam[c] = lam_next[c] + fma(arho, iv, -fma(ax, vx, ay * vy));
+    lam[(size_t)n + c] = lam_next[(size_t)n + c] + ax;
+    lam[2 * (size_t)n + c] = lam_next[2 * (size_t)n + c] + ay;
+    lam[3 * (size_t)n + c] = lam_next[3 * (size_t)n + c] + a3 * iv;
 }
 
 inline int ba(int n) { return block_for(n, BA); }
@@ -453,28 +576,32 @@ static int adjoint_step(const phd_mesh *mesh, const phd_adj_index *index, const 
     const phd_mesh &M = *mesh;
     const size_t n = M.n_cells, F = M.n_faces;
     double *face_adj = work;                       // [24][F]
-    double *cell_adj = face_adj + 24 * F;          // [12][n]
-    double *entry_adj = cell_adj + 12 * n;         // [4][2F]
-    double *self_adj = entry_adj + 8 * F;          // [4][n]
-    double *prim_adj = self_adj + 4 * n;           // [4][n]
-    cudaMemsetAsync(entry_adj, 0, sizeof(double) * 8 * F, stream);
-    cudaMemsetAsync(self_adj, 0, sizeof(double) * 4 * n, stream);
+    double *entry_adj = face_adj + 24 * F;         // [4][2F]
+    double *prim_part = entry_adj + 8 * F;         // [4][n]
     if (F && par->solver == PHD_EXACT)
-        k_adj_face<true><<<ga((int)F), ba((int)F), 0, stream>>>(M, *par, dt, prim, grad, face_w, lam_next, face_adj);
-    else if (F)
-        k_adj_face<false><<<ga((int)F), ba((int)F), 0, stream>>>(M, *par, dt, prim, grad, face_w, lam_next, face_adj);
-    k_adj_gather<<<ga((int)n), ba((int)n), 0, stream>>>(M, face_adj, cell_adj);
-    if (par->reconstruction == PHD_LINEAR)
-    {
-        if (tape_f64)
-            k_adj_grad<true><<<ga((int)n), ba((int)n), 0, stream>>>(M, *index, par->limiter, prim, cell_adj,
-                                                                  entry_adj, self_adj, tape_f64, tape_i32);
+        k_adj_face_exact<<<ga((int)F), ba((int)F), 0, stream>>>(M, *par, dt, prim, grad, face_w, lam_next, face_adj);
+    else if (F) {
+        const int block = (int)F < 16 * 128 * sm_count_current() ? 32 : 128, grid = grid_for_block((int)F, block);
+        const Gas64 C = gas64(par->gamma);
+        if (par->solver == PHD_HLLC)
+            k_adj_face<true><<<grid, block, 0, stream>>>(M, *par, C, dt, prim, grad, face_w, lam_next, face_adj);
         else
-            k_adj_grad<false><<<ga((int)n), ba((int)n), 0, stream>>>(M, *index, par->limiter, prim, cell_adj,
-                                                                   entry_adj, self_adj, nullptr, nullptr);
+            k_adj_face<false><<<grid, block, 0, stream>>>(M, *par, C, dt, prim, grad, face_w, lam_next, face_adj);
     }
-    k_adj_gather2<<<ga((int)n), ba((int)n), 0, stream>>>(M, *index, cell_adj, entry_adj, self_adj, prim_adj);
-    k_adj_final<<<ga((int)n), ba((int)n), 0, stream>>>(M, *index, par->gamma, cons, prim_adj, lam_next, lam);
+    const int bc = block_for((int)n, 128), gc = grid_for_block((int)n, bc);
+    if (par->reconstruction != PHD_LINEAR) {
+        k_adj_cell<false, false><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part,
+                                                        nullptr, nullptr);
+        k_adj_final<false><<<gc, bc, 0, stream>>>(M, *index, par->gamma, cons, prim_part, entry_adj, lam_next, lam);
+    } else {
+        if (tape_f64)
+            k_adj_cell<true, true><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part,
+                                                          tape_f64, tape_i32);
+        else
+            k_adj_cell<true, false><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part,
+                                                           nullptr, nullptr);
+        k_adj_final<true><<<gc, bc, 0, stream>>>(M, *index, par->gamma, cons, prim_part, entry_adj, lam_next, lam);
+    }
     return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
 }
 

@@ -207,8 +207,9 @@ PHD_HD __forceinline__ void gizmo64(double sl, double sr, double ci, double cj, 
 }
 
 // One side of temporal (add_temporal): X the limited spatial state, v the cell's velocity in
-// the states' frame; the state reverts to X where density or pressure would turn negative.
-PHD_HD __forceinline__ void half_step64(double *X, const double *p, const double *g, const double *v, double gamma,
+// the states' frame; the state reverts to X where density or pressure would turn negative
+// (returns true).
+PHD_HD __forceinline__ bool half_step64(double *X, const double *p, const double *g, const double *v, double gamma,
                                         double dt, bool &ok) {
     const double y = f64_rcp(p[0], ok), gp = gamma * p[3];
     double x0 = X[0], x1 = X[1] - f64_div_by(dt * g[6], p[0], y, ok), x2 = X[2] - f64_div_by(dt * g[7], p[0], y, ok),
@@ -221,12 +222,12 @@ PHD_HD __forceinline__ void half_step64(double *X, const double *p, const double
         x1 = x1 - dv * g[2 + k];
         x2 = x2 - dv * g[4 + k];
     }
-    if (!(f64_neg(x0) || f64_neg(x3))) {
-        X[0] = x0;
-        X[1] = x1;
-        X[2] = x2;
-        X[3] = x3;
-    }
+    if (f64_neg(x0) || f64_neg(x3)) return true;
+    X[0] = x0;
+    X[1] = x1;
+    X[2] = x2;
+    X[3] = x3;
+    return false;
 }
 
 // What a face reads.
