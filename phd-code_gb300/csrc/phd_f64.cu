@@ -7,6 +7,7 @@
 #include "phd_physics.cuh"
 #include "phd_ref.cuh"
 #include "phd_face64.cuh"
+#include "phd_exact64.cuh"
 
 namespace phd {
 
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(128) k_states(const __grid_constant__ phd_mesh
 // compute_fluxes by itself (the plugin's stage).
 template <int SOLVER>
 __global__ void __launch_bounds__(128) k_riemann(const __grid_constant__ phd_mesh M, const __grid_constant__ Gas64 C,
-                                                 int boost, int max_iter, const double *__restrict__ left,
+                                                 const __grid_constant__ Exact64 X, int boost, int max_iter, const double *__restrict__ left,
                                                  const double *__restrict__ right, const double *__restrict__ face_w,
                                                  double *__restrict__ flux, phd_clock *clk) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -638,7 +639,11 @@ __global__ void __launch_bounds__(128) k_riemann(const __grid_constant__ phd_mes
         big = f64_magmax(big, w[k]);
     }
     bool ok = false, failed = false;
-    if (SOLVER != PHD_EXACT && big < F64_FACE_MAX && C.ok) ok = hll64<SOLVER == PHD_HLLC>(L, R, nrm, w, C, boost != 0, f);
+    if (big < F64_FACE_MAX && C.ok) {
+        if (SOLVER == PHD_EXACT) ok = exact64_flux(L, R, nrm, w, X, max_iter, f, &failed);
+        else ok = hll64<SOLVER == PHD_HLLC>(L, R, nrm, w, C, boost != 0, f);
+    }
+    if (!ok) failed = false;
     if (!ok) riemann_flux<double, 2>(SOLVER, L, R, nrm, w, C.g, boost != 0, max_iter, f, &failed);
     if (failed) set_status(clk, PHD_STATUS_RIEMANN_NONCONVERGED);
 #pragma unroll
@@ -697,7 +702,8 @@ __device__ __noinline__ int face_flux_plain(const phd_mesh *M, const phd_params 
 // velocities by themselves -> 359 us, 1106 + 33 -> 390 FP64 instructions per warp.
 template <int SOLVER>
 __global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ phd_mesh M, const __grid_constant__ phd_params P,
-                                                   const __grid_constant__ Gas64 C, const double *__restrict__ prim,
+                                                   const __grid_constant__ Gas64 C, const __grid_constant__ Exact64 X,
+                                                   const double *__restrict__ prim,
                                                    const double *__restrict__ grad, const double *__restrict__ w,
                                                    double *__restrict__ face_w, double *__restrict__ flux,
                                                    phd_clock *clk) {
@@ -729,11 +735,9 @@ __global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ phd_m
     ok = states64(A, C, dt_half, boost, linear, P.gizmo != 0, L, R) && ok;
     int status = 0;
     if (SOLVER == PHD_EXACT) {
-        if (ok) {
-            bool failed = false;
-            exact_flux<double, 2>(L, R, nrm, A.w, C.g, P.exact_max_iter, f, &failed);
-            if (failed) status = PHD_STATUS_RIEMANN_NONCONVERGED;
-        }
+        bool failed = false;
+        ok = ok && exact64_flux(L, R, nrm, A.w, X, P.exact_max_iter, f, &failed);
+        if (failed) status = PHD_STATUS_RIEMANN_NONCONVERGED;
     } else {
         ok = hll64<SOLVER == PHD_HLLC>(L, R, nrm, A.w, C, boost, f) && ok;
     }
@@ -1073,12 +1077,13 @@ inline void launch_face_flux(const phd_mesh &M, const phd_params &P, const doubl
     // a warp's grain
     const int block = M.n_faces < 16 * 128 * sm_count_current() ? 32 : 128, grid = grid_for_block(M.n_faces, block);
     const Gas64 C = gas64(P.gamma);
+    const Exact64 X = exact64(P.gamma);
     if (P.solver == PHD_HLL)
-        k_face_flux<PHD_HLL><<<grid, block, 0, stream>>>(M, P, C, prim, grad, w, face_w, flux, clk);
+        k_face_flux<PHD_HLL><<<grid, block, 0, stream>>>(M, P, C, X, prim, grad, w, face_w, flux, clk);
     else if (P.solver == PHD_HLLC)
-        k_face_flux<PHD_HLLC><<<grid, block, 0, stream>>>(M, P, C, prim, grad, w, face_w, flux, clk);
+        k_face_flux<PHD_HLLC><<<grid, block, 0, stream>>>(M, P, C, X, prim, grad, w, face_w, flux, clk);
     else
-        k_face_flux<PHD_EXACT><<<grid, block, 0, stream>>>(M, P, C, prim, grad, w, face_w, flux, clk);
+        k_face_flux<PHD_EXACT><<<grid, block, 0, stream>>>(M, P, C, X, prim, grad, w, face_w, flux, clk);
 }
 
 inline int launch_status() {
@@ -1146,12 +1151,13 @@ int phd_riemann_f64(const phd_mesh *mesh, int32_t solver, double gamma, int32_t 
     if (mesh->n_faces == 0) return PHD_OK;
     const int block = block_for(mesh->n_faces, 128), grid = grid_for_block(mesh->n_faces, block);
     const Gas64 C = gas64(gamma);
+    const Exact64 X = exact64(gamma);
     if (solver == PHD_HLL)
-        k_riemann<PHD_HLL><<<grid, block, 0, stream>>>(*mesh, C, boost, exact_max_iter, left, right, face_w, flux, clk);
+        k_riemann<PHD_HLL><<<grid, block, 0, stream>>>(*mesh, C, X, boost, exact_max_iter, left, right, face_w, flux, clk);
     else if (solver == PHD_HLLC)
-        k_riemann<PHD_HLLC><<<grid, block, 0, stream>>>(*mesh, C, boost, exact_max_iter, left, right, face_w, flux, clk);
+        k_riemann<PHD_HLLC><<<grid, block, 0, stream>>>(*mesh, C, X, boost, exact_max_iter, left, right, face_w, flux, clk);
     else
-        k_riemann<PHD_EXACT><<<grid, block, 0, stream>>>(*mesh, C, boost, exact_max_iter, left, right, face_w, flux, clk);
+        k_riemann<PHD_EXACT><<<grid, block, 0, stream>>>(*mesh, C, X, boost, exact_max_iter, left, right, face_w, flux, clk);
     return launch_status();
 }
 
