@@ -76,8 +76,9 @@ __device__ __forceinline__ double div_ieee(double a, double b, bool &ok) {
     return div_seeded(a, b, rcp_seed(b, ok), ok);
 }
 
-// sqrt(a); clears ok for zero, negative and out-of-window radicands.
-__device__ __forceinline__ double sqrt_ieee(double a, bool &ok) {
+// 1/sqrt(a) to within 0.6 units of the last place; clears ok for zero, negative and
+// out-of-window radicands.
+__device__ __forceinline__ double rsqrt_seed(double a, bool &ok) {
     const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
     ok = ok && (hi - F64_DEN_LO < F64_DEN_SPAN);
     // a = 4^k (bh + bl), bh in [1, 4)
@@ -103,12 +104,15 @@ __device__ __forceinline__ double sqrt_ieee(double a, bool &ok) {
     const unsigned long long y = (unsigned long long)(Y10 + 512) >> 10;
     const int k = (ex - (int)odd) >> 1;
     const unsigned yh = (unsigned)(y >> 32) + (unsigned)((1021 - k) << 20);
-    const double ys = __hiloint2double((int)yh, (int)(unsigned)y);
-    const double s0 = __dmul_rn(a, ys);
-    const double r = __fma_rn(-s0, s0, a);
-    return __fma_rn(r, __hiloint2double((int)(yh - (1u << 20)), (int)(unsigned)y), s0);
+    return __hiloint2double((int)yh, (int)(unsigned)y);
 }
 
+// sqrt(a) from its seed.
+__device__ __forceinline__ double sqrt_ieee(double a, bool &ok) {
+    const double y = rsqrt_seed(a, ok), s0 = __dmul_rn(a, y);
+    const double r = __fma_rn(-s0, s0, a);
+    return __fma_rn(r, __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y)), s0);
+}
 #endif
 
 // ---- bits: comparisons, signs and halving off the FP64 pipe (finite operands) ---------

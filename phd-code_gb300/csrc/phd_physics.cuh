@@ -8,6 +8,7 @@
 // Field order: prim [rho, v_0..v_{DIM-1}, p], flux [mass, mom_0.., energy].
 #pragma once
 #include "phd_common.cuh"
+#include "phd_fp64.cuh"
 
 namespace phd {
 
@@ -193,28 +194,17 @@ PHD_HD __forceinline__ double ex_get_pstar(double dl, double ul, double pl, doub
 // evaluation at p* cost as much as the iteration itself; all three are trimmed:
 //  * gamma-only constants (2/(g-1), 2/(g+1), (g-1)/(g+1), (g-1)/2, z = (g-1)/(2g),
 //    1/z) come from the host (ExGas64);
-//  * (1 + d)^z for |d| <= 1/64 is the binomial series sum_{k=0..8} C(z,k) d^k: for
-//    0 < z < 1, |C(z,k)| <= z/k, so the dropped tail is below (1/9)(1/64)^9 / (1 - 1/64)
-//    < 1e-17 relative -- FP64 rounding level;
-//  * b^(1/z) in the two-rarefaction guess is a product of squarings when 1/z =
+//  * the powers (p/p_K)^z come from 64-bit fixed point (phd_fp64.cuh), the reciprocals and
+//    reciprocal square roots from FP32 / integer seeds: no FP64 instruction in any of them, and
+//    within 0.6 units of the last place;
+//  * b^(1/z) in the FP64 two-rarefaction guess is a product of squarings when 1/z =
 //    2g/(g-1) is an integer (5 for g = 5/3, 7 for g = 1.4), else pow;
 //  * on a rarefaction side the function and its derivative share one power,
-//    (p/p_K)^((-(g+1))/(2g)) = (p/p_K)^z * (p_K/p), and each side keeps the reciprocal
-//    of the last pressure it evaluated with that power: the next evaluation multiplies
-//    the power by (p_new/p_old)^z (series) when the ratio is within 1/64 of 1;
-//  * on a shock side s(p) = sqrt(A_K/(p + B_K)) takes one division and gives
-//    1/(p + B_K) = s^2 d (g+1)/2 without a second one; the final evaluation at p*
-//    continues from the last Newton point, s(p*) = s(p_old) (1 + e)^(-1/2),
-//    e = (p* - p_old)/(p_old + B_K), by its binomial series (six terms for
-//    |e| <= 2^-12: tail below 1e-19);
-//  * one reciprocal of the iterate per Newton step serves both sides, the shock-branch
-//    guess takes one division and one square root per side, and the convergence test
-//    2|dp|/(p_new + p_old) <= TOL is evaluated as 2|dp| <= TOL |p_new + p_old|;
-//  * on the device every FP64 reciprocal and reciprocal square root of the iteration
-//    is the hardware approximation (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64) refined
-//    by two Newton-Raphson steps (ex_rcp, ex_rsqrt): full FP64 precision for the
-//    positive normal arguments the iteration takes, in a few fused multiply-adds
-//    instead of the correctly rounded division and square root sequences.
+//    (p/p_K)^((-(g+1))/(2g)) = (p/p_K)^z * (p_K/p); on a shock side one reciprocal root,
+//    s(p) = sqrt(A_K/(p + B_K)), gives 1/(p + B_K) = s^2 d (g+1)/2 too;
+//  * one reciprocal of the iterate per Newton step serves both sides, the convergence test
+//    2|dp|/(p_new + p_old) <= TOL is evaluated as 2|dp| <= TOL |p_new + p_old|, and
+//    comparisons run on the integer pipe.
 // Results agree with ex_get_pstar to FP64 rounding of the guess (the converged p*
 // within 1e-12 relative; iteration counts can differ by one only where the relative
 // change sits within rounding of TOL).
@@ -228,7 +218,6 @@ PHD_HD __forceinline__ double ex_get_pstar(double dl, double ul, double pl, doub
 struct ExGas64 {
     double two_gm1, two_gp1, gm1_gp1, gm1_2, gp1_2, z, inv_z;
     int n_inv_z;              // 1/z when it is an integer in [1, 64], else 0
-    double c[9];              // C(z, k), k = 0..8
     double sq_two_gp1;        // sqrt(2/(g+1))
     float zf, inv_zf, two_gm1f, gm1_2f, gm1_gp1f, sq_two_gp1f;   // the same in FP32 (ex_p_guess32)
 };
@@ -252,57 +241,31 @@ inline ExGas64 ex_gas64(double gamma) {
     X.gm1_2f = (float)X.gm1_2;
     X.gm1_gp1f = (float)X.gm1_gp1;
     X.sq_two_gp1f = (float)X.sq_two_gp1;
-    X.c[0] = 1.;
-    for (int k = 1; k < 9; k++) X.c[k] = X.c[k - 1] * (X.z - double(k - 1)) / double(k);
     return X;
 }
 
-// 1/x and 1/sqrt(x) for positive normal x: on the device the hardware approximations
-// refined by two Newton-Raphson steps, y <- y (2 - x y) and y <- y (3 - x y^2) / 2 (each
-// squares the relative error, so the approximations' error reaches FP64 rounding),
-// written as a small correction added to y, y + y e with e = 1 - x y, resp.
-// e = 1/2 - (x/2) y^2, formed by fused multiply-adds so that the last rounding falls on
-// the correction; on the host (the check program) IEEE division and square root.
+// 1/x and 1/sqrt(x) for positive normal x: the seeds of phd_fp64.cuh, and outside their window
+// (no state of the iteration lies there) the plain operations.
 PHD_HD __forceinline__ double ex_rcp(double x) {
-#ifdef __CUDA_ARCH__
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double e = fma(-x, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-x, y, 1.0);
-    return fma(y, e, y);
-#else
-    return 1.0 / x;
-#endif
+    bool ok = true;
+    const double y = f64_rcp(x, ok);
+    return ok ? y : 1.0 / x;
 }
 
 PHD_HD __forceinline__ double ex_rsqrt(double x) {
 #ifdef __CUDA_ARCH__
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double h = 0.5 * x;
-    double e = fma(-h * y, y, 0.5);
-    y = fma(y, e, y);
-    e = fma(-h * y, y, 0.5);
-    return fma(y, e, y);
-#else
-    return 1.0 / sqrt(x);
+    bool ok = true;
+    const double y = rsqrt_seed(x, ok);
+    if (ok) return y;
 #endif
+    return 1.0 / sqrt(x);
 }
 
-constexpr double EX_NEAR_ONE = 0.015625;
-
-// (1 + d)^z, |d| <= 1/64
-PHD_HD __forceinline__ double ex_pow_near_one(const ExGas64 &X, double d) {
-    double s = X.c[8];
-#pragma unroll
-    for (int k = 7; k >= 0; k--) s = fma(s, d, X.c[k]);
-    return s;
-}
-
-// q^z: the series near 1, else pow
+// q^z in fixed point; else pow
 PHD_HD __forceinline__ double ex_pow_z(const ExGas64 &X, double q) {
-    return (fabs(q - 1.) <= EX_NEAR_ONE) ? ex_pow_near_one(X, q - 1.) : pow(q, X.z);
+    bool ok = log2_ok(q);
+    const double p = exp2_fix(log2_fix(q), X.z, ok);
+    return ok ? p : pow(q, X.z);
 }
 
 // b^(1/z): squarings for an integer exponent, else pow
@@ -316,11 +279,6 @@ PHD_HD __forceinline__ double ex_pow_inv_z(const ExGas64 &X, double b) {
         if (n) x *= x;
     }
     return r;
-}
-
-// (1 + e)^(-1/2), |e| <= 2^-12
-PHD_HD __forceinline__ double ex_rsqrt_near_one(double e) {
-    return fma(fma(fma(fma(fma(-63. / 256., e, 35. / 128.), e, -5. / 16.), e, 3. / 8.), e, -.5), e, 1.);
 }
 
 // ex_p_guess with the gamma constants of X: PVRS, then the two-rarefaction (TRRS) or
@@ -369,44 +327,30 @@ __device__ __forceinline__ float ex_p_guess32(float dl, float ul, float pl, floa
 #endif
 
 struct ExSide {
-    double d, p, c, Bk;
-    double inv_cd;            // 1/(c d); 0 until first needed
-    double inv_ref, qz_ref;   // 1/p and (p/p_K)^z of the last rarefaction evaluation (inv_ref 0: none)
-    double ps_ref, s_ref, u_ref;  // p, s(p) and 1/(p + B_K) of the last shock evaluation (s_ref 0: none)
+    double d, p, Bk, kc, inv_p, inv_cd;   // kc = 2 c / (g - 1)
 };
 
-PHD_HD __forceinline__ double ex_side_power(ExSide &S, const ExGas64 &X, double p_old) {
-    const double r = fma(p_old, S.inv_ref, -1.);
-    if (fabs(r) <= EX_NEAR_ONE) return S.qz_ref * ex_pow_near_one(X, r);
-    return ex_pow_z(X, p_old * ex_rcp(S.p));
+PHD_HD __forceinline__ ExSide ex_side(double d, double p, double c, const ExGas64 &X) {
+    return ExSide{d, p, p * X.gm1_gp1, c * X.two_gm1, ex_rcp(p), ex_rcp(c * d)};
 }
 
 // f_K(p_old) and f_K'(p_old) of ex_p_func / ex_p_func_deriv; inv_pold = 1 / p_old
-PHD_HD __forceinline__ void ex_side_eval(ExSide &S, const ExGas64 &X, double p_old, double inv_pold, double &f,
+PHD_HD __forceinline__ void ex_side_eval(const ExSide &S, const ExGas64 &X, double p_old, double inv_pold, double &f,
                                          double &df) {
-    if (p_old <= S.p) {
-        const double qz = ex_side_power(S, X, p_old);
-        S.inv_ref = inv_pold;
-        S.qz_ref = qz;
-        if (S.inv_cd == 0.) S.inv_cd = ex_rcp(S.c * S.d);
-        f = (S.c * X.two_gm1) * (qz - 1.);
+    if (f64_le(p_old, S.p)) {
+        const double qz = ex_pow_z(X, p_old * S.inv_p);
+        f = S.kc * (qz - 1.);
         df = (qz * (S.p * inv_pold)) * S.inv_cd;
     } else {
-        const double s = X.sq_two_gp1 * ex_rsqrt(S.d * (p_old + S.Bk));
-        const double u = ((s * s) * S.d) * X.gp1_2;         // 1/(p_old + B_K)
-        S.ps_ref = p_old;
-        S.s_ref = s;
-        S.u_ref = u;
-        f = (p_old - S.p) * s;
-        df = s * (1. - (.5 * (p_old - S.p)) * u);
+        const double s = X.sq_two_gp1 * ex_rsqrt(S.d * (p_old + S.Bk)), dp = p_old - S.p;
+        f = dp * s;
+        df = s * fma(-.5 * dp, ((s * s) * S.d) * X.gp1_2, 1.);
     }
 }
 
 // f_K(p) alone (the final evaluation at p*)
-PHD_HD __forceinline__ double ex_side_f(ExSide &S, const ExGas64 &X, double p) {
-    if (p <= S.p) return (S.c * X.two_gm1) * (ex_side_power(S, X, p) - 1.);
-    const double e = (p - S.ps_ref) * S.u_ref;
-    if (S.s_ref != 0. && fabs(e) <= 0.000244140625) return (p - S.p) * (S.s_ref * ex_rsqrt_near_one(e));
+PHD_HD __forceinline__ double ex_side_f(const ExSide &S, const ExGas64 &X, double p) {
+    if (f64_le(p, S.p)) return S.kc * (ex_pow_z(X, p * S.inv_p) - 1.);
     return (p - S.p) * (X.sq_two_gp1 * ex_rsqrt(S.d * (p + S.Bk)));
 }
 
@@ -417,21 +361,29 @@ PHD_HD __forceinline__ double ex_get_pstar_lean(double dl, double ul, double pl,
                                                 float guess32 = -1.f) {
     // guess32 > 0: the FP32 path's guess, and the side functions at p* linearised
     const double TOL = 1.0e-6;
-    ExSide Ls{dl, pl, cl, pl * X.gm1_gp1, 0., 0., 0., 0., 0., 0.};
-    ExSide Rs{dr, pr, cr, pr * X.gm1_gp1, 0., 0., 0., 0., 0., 0.};
+    const ExSide Ls = ex_side(dl, pl, cl, X), Rs = ex_side(dr, pr, cr, X);
+    const double du = ur - ul;
     const bool f32 = guess32 > 0.f && guess32 < INFINITY;
-    double p_old = f32 ? double(guess32) : ex_p_guess_lean(dl, ul, pl, cl, dr, ur, pr, cr, X);
+    double p_old;
+#ifdef __CUDA_ARCH__
+    if (f32) p_old = widen_f32(guess32);
+    else
+#endif
+    p_old = f32 ? double(guess32) : ex_p_guess_lean(dl, ul, pl, cl, dr, ur, pr, cr, X);
     double p_new = p_old;
     for (int it = 0; it < max_iter; it++) {
         double fl, fr, dfl, dfr;
-        const double inv_pold = (p_old <= pl || p_old <= pr) ? ex_rcp(p_old) : 0.;
+        const double inv_pold = ex_rcp(p_old);
         ex_side_eval(Ls, X, p_old, inv_pold, fl, dfl);
         ex_side_eval(Rs, X, p_old, inv_pold, fr, dfr);
-        p_new = p_old - ((((fl + fr) + ur) - ul) * ex_rcp(dfl + dfr));
-        const double sum = p_new + p_old;
-        if (2. * fabs(p_new - p_old) <= TOL * fabs(sum) && sum != 0.) {
+        p_new = p_old - ((fl + fr) + du) * ex_rcp(dfl + dfr);
+        const double sum = p_new + p_old, dp = p_new - p_old;
+        // 2 |dp| <= TOL |sum|, sum not zero, by the bits (a NaN's are above infinity's)
+        const unsigned long long m = 0x7fffffffffffffffull, inf = 0x7ff0000000000000ull;
+        const unsigned long long bd = (unsigned long long)f64_bits(dp) & m,
+                                 bs = (unsigned long long)f64_bits((0.5 * TOL) * sum) & m;
+        if (bd <= bs && bs != 0 && bs <= inf) {
             if (f32) {
-                const double dp = p_new - p_old;
                 fl_star = fma(dfl, dp, fl);
                 fr_star = fma(dfr, dp, fr);
             } else {
@@ -440,7 +392,8 @@ PHD_HD __forceinline__ double ex_get_pstar_lean(double dl, double ul, double pl,
             }
             return p_new;
         }
-        if (p_new < 0.) p_new = TOL;
+        if (((unsigned long long)f64_bits(p_new) & m) > inf) break;    // a NaN stays one
+        if (f64_bits(p_new) < 0) p_new = TOL;
         p_old = p_new;
     }
     *failed = true;
@@ -484,11 +437,21 @@ PHD_HD __forceinline__ void exact_flux(const T *L, const T *R, const T *n, const
 #else
         const float g32 = -1.f;
 #endif
+#ifdef __CUDA_ARCH__
+        // FP32 <-> FP64 by integer operations: the conversion instruction runs at the FP64 rate
+        const double vl = widen_f32(float(vnl)), vr = widen_f32(float(vnr));
+        const double p_star_d = ex_get_pstar_lean(widen_f32(float(_dl)), vl, widen_f32(float(_pl)), widen_f32(float(cl)),
+                                                  widen_f32(float(_dr)), vr, widen_f32(float(_pr)), widen_f32(float(cr)),
+                                                  *X, max_iter, failed, fl_d, fr_d, g32);
+        p_star = T(narrow_f64(p_star_d));
+        u_star = T(narrow_f64(0.5 * (((vl + vr) + fr_d) - fl_d)));
+#else
         const double p_star_d = ex_get_pstar_lean(double(_dl), double(vnl), double(_pl), double(cl),
                                                   double(_dr), double(vnr), double(_pr), double(cr), *X, max_iter,
                                                   failed, fl_d, fr_d, g32);
         p_star = T(p_star_d);
         u_star = T(0.5 * (((double(vnl) + double(vnr)) + fr_d) - fl_d));
+#endif
     }
     int kind;            // 0: left data, 1: right data, 2: sampled (d, p, velocity shift)
     T _d = T(0), _p = T(0), ushift = T(0);
