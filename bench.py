@@ -299,7 +299,7 @@ def run_ours(args, rank, world):
     for e in marks:
         e.record()
     torch.cuda.synchronize()
-    launch_cfg = "default (256 threads, one per item)"
+    launch_cfg = "default (shapes by size)"
     if st.precision == "fp32" and not args.no_tune:
         from phd_code_gb300.autotune import tune
         lch, _ = tune(st)

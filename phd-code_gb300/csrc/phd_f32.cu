@@ -1156,6 +1156,30 @@ inline int grid_for(int n, int block, int cap) {
     return (cap > 0 && g > cap) ? cap : (g > 0 ? g : 1);
 }
 
+// The launch shapes of a step that brings none.  The gradient and update kernels wait for
+// dependent loads and take persistent blocks filling every SM once (64 registers: 4 x 256
+// threads; 40: 4 x 384), each going over its share of the cells: the blocks of a last, nearly
+// empty wave and their starts fall away.  Measured at 1.05M cells against one cell per thread in
+// blocks of 256: gradients 65.0 -> 58.8 us (79.7 -> 73.6 without records), update 55.7 -> 45.5;
+// at 0.26M 22.0 -> 20.4 and 23.0 -> 20.4.  Up to 1.5 rounds of the gradients' threads (233,000
+// cells, one round of the update's) the blocks of one cell a thread stay: a started second
+// round would cost the persistent ones a whole one (0.2M cells: 38.8 against 42.8 us a step).
+// The face kernel takes small blocks, which leave no SM idle at the end, and two faces
+// a thread where there are several waves of them: 63.5 -> 55.7 us at 3.1M faces, 20.5 -> 18.5
+// at 0.8M.  The exact solver's, long and uneven, takes blocks of one warp (a step at 1M cells 742 ->
+// 668 us, at 0.2M 172 -> 156, against blocks of 256).
+inline phd_launch default_launch(const phd_mesh &M, int solver) {
+    const int sms = sm_count_current();
+    phd_launch L = {256, 128, 256, 0, 0, 0, 1, 1, 1};
+    if (M.n_cells > 1536 * sms) {
+        L.grid_cap_grad = L.grid_cap_update = 4 * sms;
+        if (M.n_cells > 2048 * sms) L.block_update = 384;   // up to there two even rounds of 1024 threads
+    }
+    if (solver == PHD_EXACT) L.block_face = 32;
+    else if (M.n_faces > 2 * 1280 * sms) L.items_face = 2;
+    return L;
+}
+
 inline bool block_ok(int b) { return b >= 32 && b <= 512 && (b % 32) == 0; }
 
 // items per thread: 0 (default) or 1 -> 1, 2, 4
@@ -1302,8 +1326,10 @@ int phd_step_f32_batched(const phd_mesh *mesh, const phd_geom32 *geo, const phd_
     if ((reinterpret_cast<uintptr_t>(cellrec) & 31u) != 0) return PHD_ERR_ARG;    // 256-bit loads
     if (par->solver < PHD_HLL || par->solver > PHD_EXACT) return PHD_ERR_ARG;
     if (n_runs < 1 || (n_runs > 1 && !cell_run)) return PHD_ERR_ARG;
-    phd_launch L = {B32, B32, B32, 0, 0, 0, 1, 1, 1};
-    if (launch) {
+    phd_launch L;
+    if (!launch) {
+        L = default_launch(*mesh, par->solver);
+    } else {
         if (!block_ok(launch->block_grad) || !block_ok(launch->block_face) || !block_ok(launch->block_update) ||
             launch->block_face > FACE_MAX_BLOCK || !items_ok(launch->items_grad) || !items_ok(launch->items_face) ||
             !items_ok(launch->items_update))
