@@ -452,6 +452,19 @@ int phd_step_f32_batched(const phd_mesh *mesh, const phd_geom32 *geo, const phd_
                          float *flux4, phd_clock *clocks, int32_t n_runs,
                          const int32_t *cell_run, cudaStream_t stream, cudaEvent_t *marks);
 
+/* n_steps steps of phd_step_f32_batched (without marks), the conserved totals going back and
+ * forth between cons and cons_other: the newest are in cons when n_steps is even, else in
+ * cons_other.  One call where a host loop would pay its own cost per step. */
+int phd_steps_f32(const phd_mesh *mesh, const phd_geom32 *geo, const phd_params *par,
+                  int32_t moving, const phd_launch *launch, float *prim4, double *cons,
+                  double *cons_other, float *cellrec, float *w2, float *flux4, phd_clock *clocks,
+                  int32_t n_runs, const int32_t *cell_run, int32_t n_steps, cudaStream_t stream);
+
+/* The same for phd_step_f64. */
+int phd_steps_f64(const phd_mesh *mesh, const phd_params *par, int32_t moving, double *prim,
+                  double *cons, double *cons_other, double *grad, double *w, double *face_w,
+                  double *flux, phd_clock *clk, int32_t n_steps, cudaStream_t stream);
+
 /* The same step with four caller-created events recorded on the stream around its
  * three stages (before gradients, before the face kernel, before the update, after),
  * so a caller can time each kernel inside a timed run; marks may be NULL. */

@@ -142,6 +142,9 @@ SIGNATURES = {
     "phd_load_mesh_f32": ([_PM, C.POINTER(PhdHandover32), C.POINTER(PhdParams), C.POINTER(PhdGeom32Out), _vp, _vp,
                            _vp, _vp, _vp, _vp], C.c_int),
     "phd_periodic_twins": ([_PM, _i32, _f64, _f64, _vp, _vp], C.c_int),
+    "phd_steps_f32": ([_PM, _PG, _PP, _i32, C.POINTER(PhdLaunch), _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _i32,
+                       _vp], C.c_int),
+    "phd_steps_f64": ([_PM, _PP, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp], C.c_int),
     "phd_step_f64_frozen": ([_PM, _PP, _i32, _f64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp], C.c_int),
 }
 
@@ -195,7 +198,22 @@ def ptr(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
-def stream_handle(stream=None):
-    import torch
-    s = torch.cuda.current_stream() if stream is None else stream
-    return C.c_void_p(s.cuda_stream)
+_raw_stream = None
+
+
+def stream_handle(stream=None, device=None):
+    """Raw handle of the stream, or of the current one of the device (an index; None: the
+    current device)."""
+    global _raw_stream
+    if stream is not None:
+        return C.c_void_p(stream.cuda_stream)
+    if _raw_stream is None:
+        import torch
+        torch.cuda.current_stream()               # initialises CUDA, or raises
+        raw, cur = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        # the Stream object that torch.cuda.current_stream() builds takes 5 us, the handle 0.3
+        if raw and cur:
+            _raw_stream = lambda d: raw(cur() if d is None else d)
+        else:
+            _raw_stream = lambda d: torch.cuda.current_stream(d).cuda_stream
+    return C.c_void_p(_raw_stream(device))

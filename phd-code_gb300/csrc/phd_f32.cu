@@ -1391,6 +1391,20 @@ int phd_step_f32_batched(const phd_mesh *mesh, const phd_geom32 *geo, const phd_
     return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
 }
 
+int phd_steps_f32(const phd_mesh *mesh, const phd_geom32 *geo, const phd_params *par, int32_t moving,
+                  const phd_launch *launch, float *prim4, double *cons, double *cons_other, float *cellrec, float *w2,
+                  float *flux4, phd_clock *clocks, int32_t n_runs, const int32_t *cell_run, int32_t n_steps,
+                  cudaStream_t stream) {
+    if (n_steps < 0) return PHD_ERR_ARG;
+    for (int k = 0; k < n_steps; k++) {
+        const int rc = phd_step_f32_batched(mesh, geo, par, moving, launch, prim4, (k & 1) ? cons_other : cons,
+                                            (k & 1) ? cons : cons_other, cellrec, w2, flux4, clocks, n_runs, cell_run,
+                                            stream, nullptr);
+        if (rc != PHD_OK) return rc;
+    }
+    return PHD_OK;
+}
+
 int phd_step_f32_marked(const phd_mesh *mesh, const phd_geom32 *geo, const phd_params *par, int32_t moving,
                         float *prim4, const double *cons, double *cons_next, float *cellrec, float *w2,
                         float *flux4, phd_clock *clk, cudaStream_t stream, cudaEvent_t *marks) {

@@ -1261,4 +1261,16 @@ int phd_step_f64(const phd_mesh *mesh, const phd_params *par, int32_t moving, do
                                nullptr);
 }
 
+int phd_steps_f64(const phd_mesh *mesh, const phd_params *par, int32_t moving, double *prim, double *cons,
+                  double *cons_other, double *grad, double *w, double *face_w, double *flux, phd_clock *clk,
+                  int32_t n_steps, cudaStream_t stream) {
+    if (n_steps < 0) return PHD_ERR_ARG;
+    for (int k = 0; k < n_steps; k++) {
+        const int rc = phd_step_f64(mesh, par, moving, prim, (k & 1) ? cons_other : cons, (k & 1) ? cons : cons_other, grad,
+                                    w, face_w, flux, clk, stream);
+        if (rc != PHD_OK) return rc;
+    }
+    return PHD_OK;
+}
+
 }  // extern "C"

@@ -147,6 +147,7 @@ class DeviceMesh:
             if self._csr_work.numel() < need:
                 self._csr_work = torch.empty(need + need // 8 + 16, dtype=torch.int32, device=self.device)
         self.n_cells, self.n_faces = n_cells, n_faces
+        self._shapes = None
         self._point_struct()
         return moved
 
@@ -268,14 +269,19 @@ class DeviceMesh:
         """(n_cells, n_faces) of a pinned hand-over (full or compact)."""
         return int(pinned["map"].shape[0]), int((pinned["pair_j"] if "pair_j" in pinned else pinned["pair_dj"]).shape[0])
 
+    def _upload_shapes(self):
+        return {"tag": (self.n_cells,), "type": (self.n_cells,), "map": (self.n_cells,),
+                "x": (self.dim, self.n_cells), "dcom": (self.dim, self.n_cells), "vol": (self.n_cells,),
+                "pair_i": (self.n_faces,), "pair_j": (self.n_faces,), "area": (self.n_faces,),
+                "com": (self.dim, self.n_faces), "face_ptr": (self.n_real + 1,), "area32": (self.n_faces,),
+                "ct32": (self.n_faces,), "ghost_code": (self.n_cells - self.n_real,), "pair_dj": (self.n_faces,),
+                "face32": (self.n_faces, 2)}
+
     def check_upload(self, pinned):
         """Raise unless the pinned arrays have this mesh's cell and face counts."""
-        shapes = {"tag": (self.n_cells,), "type": (self.n_cells,), "map": (self.n_cells,),
-                  "x": (self.dim, self.n_cells), "dcom": (self.dim, self.n_cells), "vol": (self.n_cells,),
-                  "pair_i": (self.n_faces,), "pair_j": (self.n_faces,), "area": (self.n_faces,),
-                  "com": (self.dim, self.n_faces), "face_ptr": (self.n_real + 1,), "area32": (self.n_faces,),
-                  "ct32": (self.n_faces,), "ghost_code": (self.n_cells - self.n_real,), "pair_dj": (self.n_faces,),
-                  "face32": (self.n_faces, 2)}
+        shapes = getattr(self, "_shapes", None)
+        if shapes is None:
+            shapes = self._shapes = self._upload_shapes()
         if "face_ptr" in pinned:
             names = ("face_ptr", "pair_j" if "pair_j" in pinned else "pair_dj", "map", "tag", "type") + \
                 (("face32",) if "face32" in pinned else ("area32", "ct32")) + \
@@ -380,8 +386,14 @@ class DeviceClock:
 
     def __init__(self, device="cuda", dt=0.0, t=0.0, t_end=0.0):
         self.device = _dev(device)
-        self.buf = torch.zeros(L.CLOCK_BYTES, dtype=torch.uint8, device=self.device)
-        self.set(dt=dt, t=t, t_end=t_end)
+        words = torch.zeros(L.CLOCK_BYTES // 8, dtype=torch.int64, device=self.device)
+        self.buf = words.view(torch.uint8)
+        if dt == 0.0 and t == 0.0 and t_end == 0.0:
+            # at rest: all zero but the CFL accumulator (infinity), filled in on the device, where
+            # a host copy would wait for the copy engine
+            words[L.PhdClock.dtmin_bits.offset // 8].fill_(0x7ff0000000000000)
+        else:
+            self.set(dt=dt, t=t, t_end=t_end)
 
     def set(self, dt=0.0, t=0.0, t_end=0.0, status=0, step=0):
         c = L.PhdClock()

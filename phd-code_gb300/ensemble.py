@@ -8,6 +8,7 @@ and each run keeps its own clock (time step from its own CFL minimum, its own ti
 is the baseline: one single-run stepper per run, launched one run after another.
 """
 import ctypes
+import operator
 
 import numpy as np
 import torch
@@ -143,8 +144,15 @@ class EnsembleStepper:
         self.cons, self.cons_next = self.cons_next, self.cons
 
     def step(self, n=1):
-        for _ in range(n):
-            self._launch_step()
+        n = max(operator.index(n), 0)
+        lch = ctypes.byref(self.launch) if self.launch is not None else None
+        L.check(L.lib().phd_steps_f32(self.dmesh.ref, ctypes.byref(self.geo), ctypes.byref(self.params),
+                                      int(self.moving), lch, L.ptr(self.prim4), L.ptr(self.cons),
+                                      L.ptr(self.cons_next), L.ptr(self.cellrec), L.ptr(self.w2),
+                                      L.ptr(self.flux4), L.ptr(self.clocks), self.n_runs, L.ptr(self.cell_run),
+                                      n, L.stream_handle()), "phd_steps_f32")
+        if n % 2:
+            self.cons, self.cons_next = self.cons_next, self.cons
 
     def capture(self, n_steps=2):
         if n_steps % 2:

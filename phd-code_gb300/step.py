@@ -11,6 +11,8 @@ Precision ``"fp64"`` is the parity mode (reference arithmetic); ``"fp32"`` runs
 reconstruction and Riemann fluxes in FP32 with FP64 conserved-state accumulation.
 """
 import ctypes
+import math
+import operator
 
 import numpy as np
 import torch
@@ -132,7 +134,7 @@ class FluxStepper:
         too small; the contents are undefined after growth."""
         if not hasattr(self, "_store"):
             self._store = {}
-        need = int(np.prod(shape))
+        need = math.prod(shape)
         store = self._store.get(name)
         if store is None and hasattr(self, name):
             store = getattr(self, name).reshape(-1)
@@ -191,6 +193,7 @@ class FluxStepper:
             self.flux4 = view("flux4", (F1, 4), f32)
             self.records = False
             self._set_geo()
+        self._handover = None
         self._graph = None
         self._graph_steps = 0
 
@@ -217,14 +220,17 @@ class FluxStepper:
         or the current ones -- and forms the ghosts' from their codes
         (``phd_ghost_positions``).  Returns the bytes copied."""
         dm, p = self.dmesh, self.params
-        main = self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
         resident = "x" not in pinned          # positions stay on the device (ghost codes come instead)
         if resident:
-            with torch.cuda.stream(main):
+            if self.stream is None:
                 xr = self._real_positions()
+            else:
+                with torch.cuda.stream(self.stream):
+                    xr = self._real_positions()
         n_new, f_new = dm.pinned_sizes(pinned)
         resized = (n_new, f_new) != (dm.n_cells, dm.n_faces)
         if resized:
+            main = self._main_stream()
             main.synchronize()            # storage may be released: nothing may still read it
             with torch.cuda.stream(main):
                 self._resize(n_new, f_new)
@@ -239,10 +245,12 @@ class FluxStepper:
             self._side2 = torch.cuda.Stream(self.device)
             self._ev = [torch.cuda.Event() for _ in range(8)]
             for e in self._ev:                        # creates the events' handles
-                e.record(main)
-        side, ev = self._side, self._ev
+                e.record(self._main_stream())
+            self._ev_handles = (ctypes.c_void_p * 8)(*(e.cuda_event for e in self._ev))
+            self._side_handles = (ctypes.c_void_p * 2)(self._side.cuda_stream, self._side2.cuda_stream)
         if compact:
-            return self._load_mesh_compact(pinned, resized, xr if resident else None, main)
+            return self._load_mesh_compact(pinned, resized, xr if resident else None)
+        side, ev, main = self._side, self._ev, self._main_stream()
         s, ss = L.stream_handle(main), L.stream_handle(side)
         out = None
         if fp32:
@@ -298,7 +306,10 @@ class FluxStepper:
             self._set_geo()
         return nbytes
 
-    def _load_mesh_compact(self, pinned, resized, xr, main):
+    def _main_stream(self):
+        return self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
+
+    def _load_mesh_compact(self, pinned, resized, xr):
         """load_mesh for the compact FP32 hand-over as one C call (phd_load_mesh_f32):
         the copies on the main stream, the derivations on two side streams while the
         face records are in flight.  xr: the real cells' device positions when the
@@ -307,9 +318,9 @@ class FluxStepper:
         nr, ng, nf = dm.n_real, dm.n_cells - dm.n_real, dm.n_faces
         nbytes = 0
         if resized:                                   # tags, types and the whole map are new
-            nbytes += dm.copy_fields(pinned, ("tag", "type", "map"), main)
+            nbytes += dm.copy_fields(pinned, ("tag", "type", "map"), self._main_stream())
         if not hasattr(dm, "_bad"):
-            dm.reset_errors(main)
+            dm.reset_errors(self._main_stream())
         packed = "pair_dj" in pinned
         n_x = pinned["pair_x"].numel() // 2 if packed else 0
         small = [k for k in ("pair_x", "face_ptr", "pair_dj", "list_len", "ghost_code")
@@ -336,32 +347,33 @@ class FluxStepper:
             stage["area32"] = self._view("area32_in", (nf,), torch.float32).data_ptr()
             stage["ct32"] = self._view("ct32_in", (nf,), torch.float32).data_ptr()
         dm.set_normals("none")
-        hp = lambda k: pinned[k].data_ptr() if k in pinned else None
-        h = L.PhdHandover32(face_ptr=hp("face_ptr"), pair_j=hp("pair_j"), area32=hp("area32"), ct32=hp("ct32"),
-                            ghost_map=None if resized else pinned["map"][nr:].data_ptr(),
-                            ghost_code=hp("ghost_code") if xr is not None else None,
-                            x=None if xr is not None else hp("x"),
-                            x_real=xr.data_ptr() if xr is not None else None, type=dm.type.data_ptr(),
-                            d_face_ptr=stage["face_ptr"], d_area32=stage.get("area32"), d_ct32=stage.get("ct32"),
-                            d_ghost_code=stage.get("ghost_code"),
-                            twin=self.twin.data_ptr(), csr_work=dm._csr_work.data_ptr(), bad=dm._bad.data_ptr(),
-                            periodic=int(dm.boundary == "periodic"), dedup_periodic=int(self.dedup_periodic),
-                            xmin=(ctypes.c_double * 2)(*dm.xmin[:2]),
-                            xmax=(ctypes.c_double * 2)(*dm.xmax[:2]),
-                            pair_dj=hp("pair_dj"), pair_x=hp("pair_x") if n_x else None, n_pair_x=n_x,
-                            d_pair_dj=stage.get("pair_dj"), d_pair_x=stage.get("pair_x"),
-                            list_len=hp("list_len"), d_list_len=stage.get("list_len"),
-                            face32=hp("face32"), d_face32=stage.get("face32"))
-        out = L.geom32(self._geo_tensors(self.handover_records), out=True)
-        events = (ctypes.c_void_p * 8)(*(e.cuda_event for e in self._ev))
-        sides = (ctypes.c_void_p * 2)(self._side.cuda_stream, self._side2.cuda_stream)
+        # the hand-over's fields of this stepper's own arrays, kept until the next _resize
+        h = getattr(self, "_handover", None)
+        if h is None:
+            h = self._handover = L.PhdHandover32(twin=self.twin.data_ptr(), xmin=(ctypes.c_double * 2)(*dm.xmin[:2]),
+                                                 xmax=(ctypes.c_double * 2)(*dm.xmax[:2]))
+            self._handover_out = L.geom32(self._geo_tensors(self.handover_records), out=True)
+        out = self._handover_out
+        h.type, h.csr_work, h.bad = dm.type.data_ptr(), dm._csr_work.data_ptr(), dm._bad.data_ptr()
+        h.periodic, h.dedup_periodic = int(dm.boundary == "periodic"), int(self.dedup_periodic)
+        for k in ("face_ptr", "pair_j", "area32", "ct32", "x", "pair_dj", "list_len", "face32"):
+            setattr(h, k, pinned[k].data_ptr() if k in pinned else None)
+        h.ghost_map = None if resized else pinned["map"].data_ptr() + 4 * nr
+        h.ghost_code = pinned["ghost_code"].data_ptr() if xr is not None and "ghost_code" in pinned else None
+        h.x_real = xr.data_ptr() if xr is not None else None
+        h.pair_x = pinned["pair_x"].data_ptr() if n_x else None
+        h.n_pair_x = n_x
+        for k in ("face_ptr", "area32", "ct32", "ghost_code", "pair_dj", "pair_x", "list_len", "face32"):
+            setattr(h, "d_" + k, stage.get(k))
         L.check(lib.phd_load_mesh_f32(dm.ref, ctypes.byref(h), ctypes.byref(self.params), ctypes.byref(out),
-                                      L.ptr(self.cons), L.ptr(self.prim4), self.clock.ptr, L.stream_handle(main),
-                                      sides, events), "phd_load_mesh_f32")
+                                      L.ptr(self.cons), L.ptr(self.prim4), self.clock.ptr,
+                                      L.stream_handle(self.stream, self.device.index), self._side_handles, self._ev_handles),
+                "phd_load_mesh_f32")
         if xr is None:
             self._x_real_valid = False
-        self.records = self.handover_records
-        self._set_geo()
+        if self.records != self.handover_records:
+            self.records = self.handover_records
+            self._set_geo()
         # what phd_load_mesh_f32 copied, counted from the arrays themselves
         nb = lambda k: pinned[k].numel() * pinned[k].element_size()
         pair_bytes = nb("pair_dj") + nb("pair_x") if packed else nb("pair_j")
@@ -400,15 +412,16 @@ class FluxStepper:
         the copy (the next step overwrites the velocities)."""
         if not self.moving:
             raise RuntimeError("generator velocities exist only in moving-mesh steps")
-        main = self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
+        main = self._main_stream()
         if getattr(self, "_fetch", None) is None:
             evs = [torch.cuda.Event() for _ in range(4)]
             for e in evs:                              # creates the events' handles
                 e.record(main)
-            self._fetch = (torch.cuda.Stream(self.device), evs, torch.cuda.Event())
-        copy_stream, evs, done = self._fetch
+            self._fetch = (torch.cuda.Stream(self.device), evs, torch.cuda.Event(),
+                           (ctypes.c_void_p * 4)(*(e.cuda_event for e in evs)))
+        copy_stream, evs, done, marks = self._fetch
         w = self.w2 if self.precision == "fp32" else self.w
-        self._launch_step(marks=(ctypes.c_void_p * 4)(*(e.cuda_event for e in evs)))
+        self._launch_step(marks=marks)
         copy_stream.wait_event(evs[1])                 # recorded after the gradient stage
         with torch.cuda.stream(copy_stream):
             host_w.copy_(w, non_blocking=True)
@@ -448,8 +461,20 @@ class FluxStepper:
 
     def step(self, n=1):
         """Launch n steps (asynchronous; read the clock or state to synchronise)."""
-        for _ in range(n):
-            self._launch_step()
+        n = max(operator.index(n), 0)
+        dm, p, s, lib = self.dmesh, self.params, L.stream_handle(self.stream), L.lib()
+        if self.precision == "fp64":
+            rc = lib.phd_steps_f64(dm.ref, ctypes.byref(p), int(self.moving), L.ptr(self.prim), L.ptr(self.cons),
+                                   L.ptr(self.cons_next), L.ptr(self.grad), L.ptr(self.w), L.ptr(self.face_w),
+                                   L.ptr(self.flux), self.clock.ptr, n, s)
+        else:
+            lch = ctypes.byref(self.launch) if self.launch is not None else None
+            rc = lib.phd_steps_f32(dm.ref, ctypes.byref(self.geo), ctypes.byref(p), int(self.moving), lch,
+                                   L.ptr(self.prim4), L.ptr(self.cons), L.ptr(self.cons_next), L.ptr(self.cellrec),
+                                   L.ptr(self.w2), L.ptr(self.flux4), self.clock.ptr, 1, None, n, s)
+        L.check(rc, "phd_steps_" + self.precision)
+        if n % 2:
+            self.cons, self.cons_next = self.cons_next, self.cons
 
     def capture(self, n_steps=2):
         """Record n_steps (even, so the double-buffered conserved state returns to the
