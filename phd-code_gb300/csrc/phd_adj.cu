@@ -181,8 +181,7 @@ __global__ void __launch_bounds__(BA) k_adj_face_exact(phd_mesh M, phd_params P,
 // HLL / HLLC: the lean reverse (phd_adjface64.cuh), the plain one for the faces it declines.
 // Bound by the FP64 pipe; held to 168 registers for 12 warps an SM (the pipe waits on 8 at 255:
 // 14.0 against 15.1 ms for 40 steps forward and backward at 128 x 128).  Measured there (50,000
-// faces, HLLC, cold caches): 317 -> 102 us at 255 registers, 2157 -> 657 FP64 instructions per
-// warp.
+// faces, HLLC, cold caches): 317 -> 67 us, 2157 -> 567 FP64 instructions per warp.
 template <bool HLLC>
 __global__ void __launch_bounds__(128, 3) k_adj_face(const __grid_constant__ phd_mesh M, const __grid_constant__ phd_params P,
                                                   const __grid_constant__ Gas64 C, double dt,

@@ -699,7 +699,7 @@ __device__ __noinline__ int face_flux_plain(const phd_mesh *M, const phd_params 
 // out of a third of the FP64 instructions.  The plain path stands in for a face with
 // unusual operands.  128 threads at 128 registers: 16 warps a SM, four times what keeps the
 // FP64 pipe fed.  Measured (160,000 cells, shear layer, HLLC): 1032 us and 35 us for the face
-// velocities by themselves -> 359 us, 1106 + 33 -> 390 FP64 instructions per warp.
+// velocities by themselves -> 291 us, 1106 + 33 -> 295 FP64 instructions per warp.
 template <int SOLVER>
 __global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ phd_mesh M, const __grid_constant__ phd_params P,
                                                    const __grid_constant__ Gas64 C, const __grid_constant__ Exact64 X,
@@ -927,9 +927,9 @@ __global__ void __launch_bounds__(BLOCK) k_time_step(phd_mesh M, const double *_
 // minimum over real cells for the next step.  The sums are cell_update_f64's, face after face
 // in list order; the loads of four faces go out together.  The time-step candidates are
 // compared in FP32 first and only the cells within its rounding of the block's smallest
-// form theirs in FP64: 16 of 106 FP64 instructions fewer in the other warps.  (Four threads a
+// form theirs in FP64: 16 FP64 instructions fewer in the other warps, 100 left.  (Four threads a
 // cell, one a field, measured no faster at 16,000 cells and 99 us against 58 at 160,000: each
-// then forms dt A by itself.)  Measured at 160,000 cells: 90.6 -> 58.4 us.
+// then forms dt A by itself.)  Measured at 160,000 cells: 90.6 -> 53.2 us.
 __global__ void __launch_bounds__(128) k_update_step(const __grid_constant__ phd_mesh M,
                                                      const __grid_constant__ phd_params P,
                                                      const double *__restrict__ flux, const double *__restrict__ cons,

@@ -1,5 +1,5 @@
-"""The FP64 kernels' quotients and square roots come from FP32 / integer seeds and three
-FP64 instructions (phd_fp64.cuh).  Against CUDA's IEEE operations: bit for bit equal on
+"""The FP64 kernels' quotients and square roots come from FP32 / integer seeds and
+integer remainders (phd_fp64.cuh).  Against CUDA's IEEE operations: bit for bit equal on
 15.5M pairs of each of six kinds, hard cases next to rounding boundaries among them; every
 operand outside the window (zeros, infinities, NaN, subnormals, negative radicands)
 declined."""
