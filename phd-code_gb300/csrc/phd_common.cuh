@@ -36,21 +36,29 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 #ifdef __CUDACC__
-// A kernel launched with programmatic stream serialization: it may be scheduled while the
-// previous kernel of the stream drains (the kernels wait for it with pdl_wait before
-// reading what it writes).  Captured into CUDA graphs as programmatic edges.
+// The kernels one call puts on a stream.  All but the first are launched with programmatic
+// stream serialization: they may be scheduled while the previous kernel of the stream drains,
+// load what the call's kernels leave alone (the mesh) and wait with pdl_wait before they
+// touch anything else.  The first waits for the stream as usual, so whatever earlier work
+// on it wrote is there for all of them.  Captured into CUDA graphs as programmatic edges.
+struct PdlQueue {
+    cudaStream_t stream;
+    bool first = true;
+};
+
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args &&...args) {
+cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, PdlQueue &q, Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
+    cfg.stream = q.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = q.first ? 0 : 1;
+    q.first = false;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 #endif

@@ -260,28 +260,6 @@ __global__ void k_prepare_csr32(phd_mesh M, const int32_t *__restrict__ twin, in
 //   f - (x + dcom) = t - dcom,  t = c + sigma r/2 n.
 // w and t of every list entry come precomputed in list order (entry_rec), so the only
 // gather left is the neighbour's primitive row.
-// The mesh rows of a cell that no kernel of the step writes (its tag, list bounds and
-// cell geometry), issued together at the start of the cell.  (Loading the next cell's
-// rows during the current one measured about 1 us slower: more live registers.)
-struct GradHead {
-    int real, e0, e1;
-    float4 gc;
-};
-
-__device__ __forceinline__ GradHead grad_head(int i, const phd_mesh &M, const float4 *__restrict__ cell_geo) {
-    GradHead h;
-    h.real = 0;
-    h.e0 = h.e1 = 0;
-    h.gc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < M.n_cells) {
-        h.real = M.tag[i] == PHD_REAL_TAG;
-        h.e0 = M.nbr_ptr[i];
-        h.e1 = M.nbr_ptr[i + 1];
-        h.gc = cell_geo[i];
-    }
-    return h;
-}
-
 // Where the list entries' gradient records come from: REC, the precomputed entry_rec in
 // list order; otherwise each entry's record is formed here from its face's records
 // (csr_face -> face_geo, face_ar) with entry_record's roundings, the same bits (a mesh
@@ -305,74 +283,111 @@ __device__ __forceinline__ float4 entry_t_of(const EntrySrc &S, int e) {
     return make_float4(0.f, 0.f, t.x, t.y);
 }
 
-template <int LIMITER, bool REC>
-__device__ __forceinline__ void grad32_cell(int i, const GradHead &H, const phd_mesh &M, const phd_params &P,
+// What a cell's gradient reads of the mesh, which no kernel of the step writes: its row or
+// its image's, and the first chunk of list entries.  Where every thread has one cell
+// (ITEMS 0) these loads go out before the wait for the previous kernel, so two of the three
+// dependent loads of a list pass while that one drains; the face and update kernels do the
+// same with their mesh rows.  On a mesh that is one wave of blocks or less the step is a
+// chain of such latencies: 15.4 -> 13.1 us at 1,000 cells, 28.2 -> 25.4 at 111,000 (HLL,
+// TESS).  Threads that loop load in place: they hide the latency behind each other, and the
+// rows kept across the wait cost registers (the update's 58 against 40).  (Loading the next
+// cell's rows during the current one measured about 1 us slower for the same reason.)
+template <bool REC>
+struct GradHead {
+    // entries in chunks of CH: all of a chunk's loads are issued before any arithmetic,
+    // so their latencies overlap (lanes past the end reload entry e0)
+    // (two entries per chunk when the records are formed here: 4 took 84 registers and
+    // ran 96 us against 76 at 1M cells)
+    static constexpr int CH = REC ? 4 : 2;
+    int c, e0, e1, nb[CH];
+    float4 gc, rw[CH];
+};
+
+// Entries eb .. eb + CH - 1: the neighbours and the gradient records.
+template <bool REC>
+__device__ __forceinline__ void grad_entries(GradHead<REC> &H, int eb, const EntrySrc &S,
+                                             const int32_t *__restrict__ csr_nbr) {
+    constexpr int CH = GradHead<REC>::CH;
+    if (REC) {
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            const int e = (eb + k < H.e1) ? eb + k : H.e0;
+            H.nb[k] = csr_nbr[e];
+            H.rw[k] = S.entry_rec[e];
+        }
+    } else {
+        int code[CH];
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            const int e = (eb + k < H.e1) ? eb + k : H.e0;
+            H.nb[k] = csr_nbr[e];
+            code[k] = S.csr_face[e];
+        }
+        float4 g[CH];
+        float2 ar[CH];
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            const int fid = code[k] < 0 ? ~code[k] : code[k];
+            const int f = (fid >= 0 && fid < S.n_faces) ? fid : 0;
+            g[k] = S.face_geo[f];
+            ar[k] = S.face_ar[f];
+        }
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            const int fid = code[k] < 0 ? ~code[k] : code[k];
+            H.rw[k] = (fid >= 0 && fid < S.n_faces) ? entry_record(g[k], ar[k], code[k] < 0)
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+}
+
+// PRE: with the first chunk.
+template <bool REC, bool PRE>
+__device__ __forceinline__ GradHead<REC> grad_head(int i, const phd_mesh &M, const EntrySrc &S,
+                                                   const int32_t *__restrict__ csr_nbr,
+                                                   const float4 *__restrict__ cell_geo) {
+    GradHead<REC> h;
+    h.c = -1;
+    h.e0 = h.e1 = 0;
+    if (i >= M.n_cells) return h;
+    // the cell's own rows go out before its tag is known: for a real cell they are the
+    // rows the gradient needs; a ghost reloads its image's
+    const bool real = M.tag[i] == PHD_REAL_TAG;
+    h.e0 = M.nbr_ptr[i];
+    h.e1 = M.nbr_ptr[i + 1];
+    h.gc = cell_geo[i];
+    h.c = i;
+    if (!real) {
+        h.c = M.map[i];
+        if (h.c < 0 || h.c >= M.n_cells) { h.c = -1; return h; }
+        h.gc = cell_geo[h.c];
+        h.e0 = M.nbr_ptr[h.c];
+        h.e1 = M.nbr_ptr[h.c + 1];
+    }
+    if (PRE && h.e0 < h.e1) grad_entries<REC>(h, h.e0, S, csr_nbr);
+    return h;
+}
+
+template <int LIMITER, bool REC, bool PRE>
+__device__ __forceinline__ void grad32_cell(int i, GradHead<REC> &H, const phd_mesh &M, const phd_params &P,
                                             int moving, const EntrySrc &S,
                                             const int32_t *__restrict__ csr_nbr,
                                             const float4 *__restrict__ cell_geo,
                                             const float4 *__restrict__ prim4, float4 *__restrict__ cellrec,
                                             float2 *__restrict__ w2, phd_clock *clk) {
-    // the cell's own rows were loaded before its tag was known: for a real cell they are
-    // the rows the gradient needs; a ghost reloads its twin's
-    const bool real = H.real;
-    float4 pc = prim4[i];
-    float4 gc = H.gc;
-    int e0 = H.e0, e1 = H.e1;
-    int c = i;
-    if (!real) {
-        c = M.map[i];
-        if (c < 0 || c >= M.n_cells) { set_status32(clk, PHD_STATUS_BAD_INDEX); return; }
-        pc = prim4[c];
-        gc = cell_geo[c];
-        e0 = M.nbr_ptr[c];
-        e1 = M.nbr_ptr[c + 1];
-    }
+    const int c = H.c, e0 = H.e0, e1 = H.e1;
+    if (c < 0) { set_status32(clk, PHD_STATUS_BAD_INDEX); return; }
+    const float4 pc = prim4[c], gc = H.gc;
     const float P0[4] = {pc.x, pc.y, pc.z, pc.w};
     float dmx[4], dmn[4], df[4][2];
 #pragma unroll
     for (int f = 0; f < 4; f++) { dmx[f] = dmn[f] = 0.f; df[f][0] = df[f][1] = 0.f; }
-    // entries in chunks of CH: all of a chunk's loads are issued before any arithmetic,
-    // so their latencies overlap (lanes past the end reload entry e0)
-    // (two entries per chunk when the records are formed here: 4 took 84 registers and
-    // ran 96 us against 76 at 1M cells)
-    constexpr int CH = REC ? 4 : 2;
+    constexpr int CH = GradHead<REC>::CH;
     for (int eb = e0; eb < e1; eb += CH) {
-        int nb[CH];
-        float4 rw[CH];
-        if (REC) {
-#pragma unroll
-            for (int k = 0; k < CH; k++) {
-                const int e = (eb + k < e1) ? eb + k : e0;
-                nb[k] = csr_nbr[e];
-                rw[k] = S.entry_rec[e];
-            }
-        } else {
-            int code[CH];
-#pragma unroll
-            for (int k = 0; k < CH; k++) {
-                const int e = (eb + k < e1) ? eb + k : e0;
-                nb[k] = csr_nbr[e];
-                code[k] = S.csr_face[e];
-            }
-            float4 g[CH];
-            float2 ar[CH];
-#pragma unroll
-            for (int k = 0; k < CH; k++) {
-                const int fid = code[k] < 0 ? ~code[k] : code[k];
-                const int f = (fid >= 0 && fid < S.n_faces) ? fid : 0;
-                g[k] = S.face_geo[f];
-                ar[k] = S.face_ar[f];
-            }
-#pragma unroll
-            for (int k = 0; k < CH; k++) {
-                const int fid = code[k] < 0 ? ~code[k] : code[k];
-                rw[k] = (fid >= 0 && fid < S.n_faces) ? entry_record(g[k], ar[k], code[k] < 0)
-                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
+        if (!PRE || eb != e0) grad_entries<REC>(H, eb, S, csr_nbr);
         float4 pj[CH];
 #pragma unroll
-        for (int k = 0; k < CH; k++) pj[k] = prim4[nb[k]];
+        for (int k = 0; k < CH; k++) pj[k] = prim4[H.nb[k]];
 #pragma unroll
         for (int k = 0; k < CH; k++) {
             if (eb + k >= e1) break;
@@ -382,8 +397,8 @@ __device__ __forceinline__ void grad32_cell(int i, const GradHead &H, const phd_
                 const float d = Pj[f] - P0[f];
                 dmx[f] = fmaxf(dmx[f], d);
                 dmn[f] = fminf(dmn[f], d);
-                df[f][0] += d * rw[k].x;
-                df[f][1] += d * rw[k].y;
+                df[f][0] += d * H.rw[k].x;
+                df[f][1] += d * H.rw[k].y;
             }
         }
     }
@@ -477,7 +492,8 @@ __device__ __forceinline__ void grad32_cell(int i, const GradHead &H, const phd_
 }
 
 // ITEMS cells per thread: a block covers blockDim * ITEMS consecutive cells, thread t
-// taking cells t, t + blockDim, ... of each tile (the autotuner picks 1, 2 or 4).
+// taking cells t, t + blockDim, ... of each tile (the autotuner picks 1, 2 or 4).  ITEMS 0:
+// one cell per thread and no loop, for grids that cover the mesh.
 template <int LIMITER, int ITEMS, bool REC>
 __global__ void __launch_bounds__(512) k_grad32(phd_mesh M, phd_params P, int moving, EntrySrc S,
                                                 const int32_t *__restrict__ csr_nbr,
@@ -485,15 +501,23 @@ __global__ void __launch_bounds__(512) k_grad32(phd_mesh M, phd_params P, int mo
                                                 const float4 *__restrict__ prim4, float4 *__restrict__ cellrec,
                                                 float2 *__restrict__ w2, phd_clock *clk) {
     pdl_launch_dependents();
+    if (ITEMS == 0) {
+        const int i = blockIdx.x * blockDim.x + threadIdx.x;
+        GradHead<REC> H = grad_head<REC, true>(i, M, S, csr_nbr, cell_geo);
+        pdl_wait();                              // prim4: written by the previous step's update
+        if (i < M.n_cells)
+            grad32_cell<LIMITER, REC, true>(i, H, M, P, moving, S, csr_nbr, cell_geo, prim4, cellrec, w2, clk);
+        return;
+    }
     const int tile = blockDim.x * ITEMS;
-    pdl_wait();                                  // prim4: written by the previous step's update
+    pdl_wait();
     for (int base = blockIdx.x * tile; base < M.n_cells; base += gridDim.x * tile) {
 #pragma unroll
         for (int k = 0; k < ITEMS; k++) {
             const int i = base + k * blockDim.x + threadIdx.x;
-            if (i < M.n_cells)
-                grad32_cell<LIMITER, REC>(i, grad_head(i, M, cell_geo), M, P, moving, S, csr_nbr, cell_geo, prim4,
-                                          cellrec, w2, clk);
+            if (i >= M.n_cells) continue;
+            GradHead<REC> H = grad_head<REC, false>(i, M, S, csr_nbr, cell_geo);
+            grad32_cell<LIMITER, REC, false>(i, H, M, P, moving, S, csr_nbr, cell_geo, prim4, cellrec, w2, clk);
         }
     }
 }
@@ -818,8 +842,17 @@ __global__ void __launch_bounds__(FACE_MAX_BLOCK, SOLVER == PHD_EXACT ? 1 : 5) k
                                                 float4 *__restrict__ flux4, phd_clock *clocks,
                                                 const int32_t *__restrict__ cell_run, const __grid_constant__ GasC GC) {
     pdl_launch_dependents();
+    if (ITEMS == 0) {
+        const int m = blockIdx.x * blockDim.x + threadIdx.x;
+        const FaceHead H = face_head(m, M, face_geo, face_ar);
+        pdl_wait();                              // cellrec / prim4, w2 and the clock: earlier kernels'
+        const float dt_run = cell_run ? 0.f : narrow_f64(clocks->dt);
+        if (m < M.n_faces)
+            face32_face<SOLVER, LINEAR, BOOST>(m, H, M, P, moving, prim4, cellrec, w2, flux4, clocks, cell_run, GC, dt_run);
+        return;
+    }
     const int tile = blockDim.x * ITEMS;
-    pdl_wait();                                  // cellrec / prim4, w2 and the clock: earlier kernels'
+    pdl_wait();
     const float dt_run = cell_run ? 0.f : narrow_f64(clocks->dt);
     for (int base = blockIdx.x * tile; base < M.n_faces; base += gridDim.x * tile) {
 #pragma unroll
@@ -839,26 +872,46 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
     e = (a - (s - bb)) + (b - bb);
 }
 
-// One cell of the update: segmented sum, FP64 totals, primitives; returns the CFL
-// candidate (INFINITY for ghosts) and the cell's run.
-// A cell's mesh rows for the update (tag and list bounds).
+// What a cell's update reads of the mesh: its list or its image's, and the first chunk of
+// its codes (loaded while the face kernel drains, as in k_grad32).
 struct UpdHead {
-    int real, e0, e1;
+    static constexpr int CH = 8;          // measured best for this kernel (CH = 1, 2, 4, 8 tried)
+    int real, c, e0, e1, code[CH];
 };
 
-__device__ __forceinline__ UpdHead upd_head(int i, const phd_mesh &M) {
+__device__ __forceinline__ void upd_codes(UpdHead &H, int eb, const int32_t *__restrict__ csr_face) {
+#pragma unroll
+    for (int k = 0; k < UpdHead::CH; k++) H.code[k] = csr_face[(eb + k < H.e1) ? eb + k : H.e0];
+}
+
+// PRE: with the first chunk.
+template <bool PRE>
+__device__ __forceinline__ UpdHead upd_head(int i, const phd_mesh &M, const int32_t *__restrict__ csr_face) {
     UpdHead h;
     h.real = 0;
+    h.c = -1;
     h.e0 = h.e1 = 0;
-    if (i < M.n_cells) {
-        h.real = M.tag[i] == PHD_REAL_TAG;
-        h.e0 = M.nbr_ptr[i];
-        h.e1 = M.nbr_ptr[i + 1];
+    if (i >= M.n_cells) return h;
+    // the cell's own list bounds go out before its tag is known (a real cell's are the
+    // ones it needs); a ghost reloads its image's
+    h.real = M.tag[i] == PHD_REAL_TAG;
+    h.e0 = M.nbr_ptr[i];
+    h.e1 = M.nbr_ptr[i + 1];
+    h.c = i;
+    if (!h.real) {
+        h.c = M.map[i];
+        if (h.c < 0 || h.c >= M.n_cells) { h.c = -1; return h; }
+        h.e0 = M.nbr_ptr[h.c];
+        h.e1 = M.nbr_ptr[h.c + 1];
     }
+    if (PRE && h.e0 < h.e1) upd_codes(h, h.e0, csr_face);
     return h;
 }
 
-__device__ __forceinline__ float update32_cell(int i, const UpdHead &H, const phd_mesh &M, const phd_params &P,
+// One cell of the update: segmented sum, FP64 totals, primitives; returns the CFL
+// candidate (INFINITY for ghosts) and the cell's run.
+template <bool PRE>
+__device__ __forceinline__ float update32_cell(int i, UpdHead &H, const phd_mesh &M, const phd_params &P,
                                                const int32_t *__restrict__ csr_face,
                                                const float4 *__restrict__ flux4,
                                                const float4 *__restrict__ cell_geo,
@@ -867,22 +920,14 @@ __device__ __forceinline__ float update32_cell(int i, const UpdHead &H, const ph
                                                const int32_t *__restrict__ cell_run, float gam) {
     const int n = M.n_cells;
     phd_clock *clk = cell_run ? clocks + cell_run[i] : clocks;
-    // the cell's own list bounds were loaded before its tag was known (a real cell's are
-    // the ones it needs); a ghost reloads its image's
+    const int c = H.c, e0 = H.e0, e1 = H.e1;
     const bool real = H.real;
-    int e0 = H.e0, e1 = H.e1;
-    const int c = real ? i : M.map[i];
-    if (c < 0 || c >= n) { set_status32(clk, PHD_STATUS_BAD_INDEX); return INFINITY; }
-    if (!real) {
-        e0 = M.nbr_ptr[c];
-        e1 = M.nbr_ptr[c + 1];
-    }
+    if (c < 0) { set_status32(clk, PHD_STATUS_BAD_INDEX); return INFINITY; }
     float hs[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
-    constexpr int CH = 8;          // measured best for this kernel (CH = 1, 2, 4, 8 tried)
+    constexpr int CH = UpdHead::CH;
     for (int eb = e0; eb < e1; eb += CH) {
-        int code[CH];
-#pragma unroll
-        for (int k = 0; k < CH; k++) code[k] = csr_face[(eb + k < e1) ? eb + k : e0];
+        if (!PRE || eb != e0) upd_codes(H, eb, csr_face);
+        const int *code = H.code;
         float4 fl[CH];
 #pragma unroll
         for (int k = 0; k < CH; k++) fl[k] = flux4[code[k] < 0 ? ~code[k] : code[k]];
@@ -950,20 +995,24 @@ __global__ void __launch_bounds__(512) k_update32(phd_mesh M, phd_params P, cons
     pdl_launch_dependents();
     const int n = M.n_cells;
     const float gam = narrow_f64(P.gamma);
-    const int tile = blockDim.x * ITEMS;
+    constexpr int K = ITEMS == 0 ? 1 : ITEMS;
+    const int tile = blockDim.x * K;
     const int stride = gridDim.x * tile;
-    const int n_iter = (n + stride - 1) / stride;     // uniform trip count: all lanes reach the shuffles
+    const int n_iter = ITEMS == 0 ? 1 : (n + stride - 1) / stride;     // uniform trip count: all lanes reach the shuffles
     float cand_all = INFINITY;
+    UpdHead H;
+    if (ITEMS == 0) H = upd_head<true>(blockIdx.x * tile + threadIdx.x, M, csr_face);
     pdl_wait();                                       // flux4: the face kernel's; the clocks
     for (int it = 0; it < n_iter; it++) {
 #pragma unroll
-        for (int k = 0; k < ITEMS; k++) {
+        for (int k = 0; k < K; k++) {
             const int i = blockIdx.x * tile + it * stride + k * blockDim.x + threadIdx.x;
             float cand = INFINITY;
             int run = 0;
             if (i < n) {
-                cand = update32_cell(i, upd_head(i, M), M, P, csr_face, flux4, cell_geo, cons, cons_next, prim4,
-                                     clocks, cell_run, gam);
+                if (ITEMS != 0) H = upd_head<false>(i, M, csr_face);
+                cand = update32_cell<ITEMS == 0>(i, H, M, P, csr_face, flux4, cell_geo, cons, cons_next, prim4, clocks, cell_run,
+                                     gam);
                 if (cell_run) run = cell_run[i];
             }
             if (!cell_run) {
@@ -1109,7 +1158,7 @@ int cells_prim_f32(const phd_mesh *mesh, const phd_params *par, const phd_geom32
 }
 
 template <int SOLVER, int ITEMS>
-void launch_face32_items(bool linear, int grid, int block, cudaStream_t s, const phd_mesh &M, const phd_params &P,
+void launch_face32_items(bool linear, int grid, int block, PdlQueue &s, const phd_mesh &M, const phd_params &P,
                          int moving, const phd_geom32 *G, const float4 *prim4, const float4 *cellrec, const float2 *w2,
                          float4 *flux4, phd_clock *clocks, const int32_t *cell_run) {
     const float4 *fg = reinterpret_cast<const float4 *>(G->face_geo);
@@ -1136,10 +1185,13 @@ void launch_face32_items(bool linear, int grid, int block, cudaStream_t s, const
 // The exact solver's face kernel is bound by the FP64 pipe and holds 120+ registers:
 // it runs one face per thread whatever the requested items.
 template <int SOLVER>
-void launch_face32(bool linear, int items, int grid, int block, cudaStream_t s, const phd_mesh &M,
+void launch_face32(bool linear, int items, int grid, int block, PdlQueue &s, const phd_mesh &M,
                    const phd_params &P, int moving, const phd_geom32 *G, const float4 *prim4, const float4 *cellrec,
                    const float2 *w2, float4 *flux4, phd_clock *clocks, const int32_t *cell_run) {
-    if (SOLVER == PHD_EXACT || items == 1)
+    if (items == 0)
+        launch_face32_items<SOLVER, 0>(linear, grid, block, s, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
+                                       cell_run);
+    else if (SOLVER == PHD_EXACT || items == 1)
         launch_face32_items<SOLVER, 1>(linear, grid, block, s, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
                                        cell_run);
     else if (items == 2)
@@ -1187,10 +1239,12 @@ inline bool items_ok(int k) { return k == 0 || k == 1 || k == 2 || k == 4; }
 inline int items_of(int k) { return k <= 1 ? 1 : k; }
 
 template <int LIMITER>
-void launch_grad32_rec(int items, int grid, int block, cudaStream_t s, const phd_mesh &M, const phd_params &P,
+void launch_grad32_rec(int items, int grid, int block, PdlQueue &s, const phd_mesh &M, const phd_params &P,
                        int moving, const EntrySrc &S, const int32_t *csr_nbr, const float4 *cg, const float4 *p4,
                        float4 *cr, float2 *w, phd_clock *clocks) {
-    if (items == 1)
+    if (items == 0)
+        launch_pdl(k_grad32<LIMITER, 0, true>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+    else if (items == 1)
         launch_pdl(k_grad32<LIMITER, 1, true>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else if (items == 2)
         launch_pdl(k_grad32<LIMITER, 2, true>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
@@ -1201,11 +1255,13 @@ void launch_grad32_rec(int items, int grid, int block, cudaStream_t s, const phd
 // without entry records (S.entry_rec null): one item per thread, the records formed
 // from the faces (the launch a freshly handed-over mesh's first step takes)
 template <int LIMITER>
-void launch_grad32(int items, int grid, int block, cudaStream_t s, const phd_mesh &M, const phd_params &P, int moving,
+void launch_grad32(int items, int grid, int block, PdlQueue &s, const phd_mesh &M, const phd_params &P, int moving,
                    const EntrySrc &S, const int32_t *csr_nbr, const float4 *cg, const float4 *p4, float4 *cr,
                    float2 *w, phd_clock *clocks) {
     if (S.entry_rec)
         launch_grad32_rec<LIMITER>(items, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+    else if (items == 0)
+        launch_pdl(k_grad32<LIMITER, 0, false>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else if (items == 1)
         launch_pdl(k_grad32<LIMITER, 1, false>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else
@@ -1226,6 +1282,94 @@ int prepare_faces32_interleaved(const phd_mesh *mesh, const float *face32, phd_g
 }  // namespace phd
 
 using namespace phd;
+
+// One step on the queue: gradients (where they or the generator velocities are needed),
+// faces, update.
+static int step_f32(const phd_mesh *mesh, const phd_geom32 *geo, const phd_params *par, int32_t moving,
+                         const phd_launch *launch, float *prim4, const double *cons, double *cons_next, float *cellrec,
+                         float *w2, float *flux4, phd_clock *clocks, int32_t n_runs, const int32_t *cell_run,
+                         PdlQueue &stream, cudaEvent_t *marks) {
+    if (!mesh || mesh->dim != 2 || !geo || !par || !prim4 || !cons || !cons_next || !flux4 || !clocks)
+        return PHD_ERR_ARG;
+    const bool linear = par->reconstruction == PHD_LINEAR;
+    if ((linear || moving) && (!cellrec || !geo->csr_nbr)) return PHD_ERR_ARG;
+    if ((linear || moving) && !geo->entry_rec && (!geo->face_geo || !geo->face_ar || !geo->csr_face))
+        return PHD_ERR_ARG;
+    if (moving && !w2) return PHD_ERR_ARG;
+    if ((reinterpret_cast<uintptr_t>(cellrec) & 31u) != 0) return PHD_ERR_ARG;    // 256-bit loads
+    if (par->solver < PHD_HLL || par->solver > PHD_EXACT) return PHD_ERR_ARG;
+    if (n_runs < 1 || (n_runs > 1 && !cell_run)) return PHD_ERR_ARG;
+    phd_launch L;
+    if (!launch) {
+        L = default_launch(*mesh, par->solver);
+    } else {
+        if (!block_ok(launch->block_grad) || !block_ok(launch->block_face) || !block_ok(launch->block_update) ||
+            launch->block_face > FACE_MAX_BLOCK || !items_ok(launch->items_grad) || !items_ok(launch->items_face) ||
+            !items_ok(launch->items_update))
+            return PHD_ERR_ARG;
+        L = *launch;
+    }
+    const int ig = items_of(L.items_grad), ifc = par->solver == PHD_EXACT ? 1 : items_of(L.items_face),
+              iu = items_of(L.items_update);
+    const phd_mesh &M = *mesh;
+    const int gc = grid_for((M.n_cells + ig - 1) / ig, L.block_grad, L.grid_cap_grad);
+    const int gf = grid_for((M.n_faces + ifc - 1) / ifc, L.block_face, L.grid_cap_face);
+    const int gu = grid_for((M.n_cells + iu - 1) / iu, L.block_update, L.grid_cap_update);
+    // one cell or face a thread, none left over: the instances that load ahead of their wait (0)
+    const int kg = ig == 1 && (long long)gc * L.block_grad >= M.n_cells ? 0 : ig;
+    const int kf = ifc == 1 && (long long)gf * L.block_face >= M.n_faces ? 0 : ifc;
+    const int ku = iu == 1 && (long long)gu * L.block_update >= M.n_cells ? 0 : iu;
+    float4 *p4 = reinterpret_cast<float4 *>(prim4);
+    float4 *cr = reinterpret_cast<float4 *>(cellrec);
+    float2 *w = reinterpret_cast<float2 *>(w2);
+    float4 *fx = reinterpret_cast<float4 *>(flux4);
+    const EntrySrc er = {reinterpret_cast<const float4 *>(geo->entry_rec), geo->csr_face,
+                         reinterpret_cast<const float4 *>(geo->face_geo), reinterpret_cast<const float2 *>(geo->face_ar),
+                         M.n_faces};
+    const float4 *cg = reinterpret_cast<const float4 *>(geo->cell_geo);
+    const int32_t *runs = n_runs > 1 ? cell_run : nullptr;
+    if (marks) cudaEventRecord(marks[0], stream.stream);
+    if (linear || moving) {
+        if (par->limiter == PHD_LIMITER_TESS)
+            launch_grad32<PHD_LIMITER_TESS>(kg, gc, L.block_grad, stream, M, *par, (int)moving, er, geo->csr_nbr, cg,
+                                            p4, cr, w, clocks);
+        else
+            launch_grad32<PHD_LIMITER_AREPO>(kg, gc, L.block_grad, stream, M, *par, (int)moving, er, geo->csr_nbr, cg,
+                                             p4, cr, w, clocks);
+    }
+    if (marks) cudaEventRecord(marks[1], stream.stream);
+    if (M.n_faces) {
+        switch (par->solver) {
+            case PHD_HLL:
+                launch_face32<PHD_HLL>(linear, kf, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx, clocks,
+                                       runs);
+                break;
+            case PHD_HLLC:
+                launch_face32<PHD_HLLC>(linear, kf, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx, clocks,
+                                        runs);
+                break;
+            default:
+                launch_face32<PHD_EXACT>(linear, kf, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx,
+                                         clocks, runs);
+                break;
+        }
+    }
+    if (marks) cudaEventRecord(marks[2], stream.stream);
+    if (ku == 0)
+        launch_pdl(k_update32<0>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
+                   cons_next, p4, clocks, runs, (int)n_runs);
+    else if (ku == 1)
+        launch_pdl(k_update32<1>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
+                   cons_next, p4, clocks, runs, (int)n_runs);
+    else if (ku == 2)
+        launch_pdl(k_update32<2>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
+                   cons_next, p4, clocks, runs, (int)n_runs);
+    else
+        launch_pdl(k_update32<4>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
+                   cons_next, p4, clocks, runs, (int)n_runs);
+    if (marks) cudaEventRecord(marks[3], stream.stream);
+    return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
+}
 
 extern "C" {
 
@@ -1316,79 +1460,9 @@ int phd_step_f32_batched(const phd_mesh *mesh, const phd_geom32 *geo, const phd_
                          float *w2, float *flux4, phd_clock *clocks, int32_t n_runs, const int32_t *cell_run,
                          cudaStream_t stream, cudaEvent_t *marks) {
     phd::NvtxRange nvtx_range("phd_step_f32");
-    if (!mesh || mesh->dim != 2 || !geo || !par || !prim4 || !cons || !cons_next || !flux4 || !clocks)
-        return PHD_ERR_ARG;
-    const bool linear = par->reconstruction == PHD_LINEAR;
-    if ((linear || moving) && (!cellrec || !geo->csr_nbr)) return PHD_ERR_ARG;
-    if ((linear || moving) && !geo->entry_rec && (!geo->face_geo || !geo->face_ar || !geo->csr_face))
-        return PHD_ERR_ARG;
-    if (moving && !w2) return PHD_ERR_ARG;
-    if ((reinterpret_cast<uintptr_t>(cellrec) & 31u) != 0) return PHD_ERR_ARG;    // 256-bit loads
-    if (par->solver < PHD_HLL || par->solver > PHD_EXACT) return PHD_ERR_ARG;
-    if (n_runs < 1 || (n_runs > 1 && !cell_run)) return PHD_ERR_ARG;
-    phd_launch L;
-    if (!launch) {
-        L = default_launch(*mesh, par->solver);
-    } else {
-        if (!block_ok(launch->block_grad) || !block_ok(launch->block_face) || !block_ok(launch->block_update) ||
-            launch->block_face > FACE_MAX_BLOCK || !items_ok(launch->items_grad) || !items_ok(launch->items_face) ||
-            !items_ok(launch->items_update))
-            return PHD_ERR_ARG;
-        L = *launch;
-    }
-    const int ig = items_of(L.items_grad), ifc = par->solver == PHD_EXACT ? 1 : items_of(L.items_face),
-              iu = items_of(L.items_update);
-    const phd_mesh &M = *mesh;
-    const int gc = grid_for((M.n_cells + ig - 1) / ig, L.block_grad, L.grid_cap_grad);
-    const int gf = grid_for((M.n_faces + ifc - 1) / ifc, L.block_face, L.grid_cap_face);
-    const int gu = grid_for((M.n_cells + iu - 1) / iu, L.block_update, L.grid_cap_update);
-    float4 *p4 = reinterpret_cast<float4 *>(prim4);
-    float4 *cr = reinterpret_cast<float4 *>(cellrec);
-    float2 *w = reinterpret_cast<float2 *>(w2);
-    float4 *fx = reinterpret_cast<float4 *>(flux4);
-    const EntrySrc er = {reinterpret_cast<const float4 *>(geo->entry_rec), geo->csr_face,
-                         reinterpret_cast<const float4 *>(geo->face_geo), reinterpret_cast<const float2 *>(geo->face_ar),
-                         M.n_faces};
-    const float4 *cg = reinterpret_cast<const float4 *>(geo->cell_geo);
-    const int32_t *runs = n_runs > 1 ? cell_run : nullptr;
-    if (marks) cudaEventRecord(marks[0], stream);
-    if (linear || moving) {
-        if (par->limiter == PHD_LIMITER_TESS)
-            launch_grad32<PHD_LIMITER_TESS>(ig, gc, L.block_grad, stream, M, *par, (int)moving, er, geo->csr_nbr, cg,
-                                            p4, cr, w, clocks);
-        else
-            launch_grad32<PHD_LIMITER_AREPO>(ig, gc, L.block_grad, stream, M, *par, (int)moving, er, geo->csr_nbr, cg,
-                                             p4, cr, w, clocks);
-    }
-    if (marks) cudaEventRecord(marks[1], stream);
-    if (M.n_faces) {
-        switch (par->solver) {
-            case PHD_HLL:
-                launch_face32<PHD_HLL>(linear, ifc, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx, clocks,
-                                       runs);
-                break;
-            case PHD_HLLC:
-                launch_face32<PHD_HLLC>(linear, ifc, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx, clocks,
-                                        runs);
-                break;
-            default:
-                launch_face32<PHD_EXACT>(linear, 1, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx,
-                                         clocks, runs);
-                break;
-        }
-    }
-    if (marks) cudaEventRecord(marks[2], stream);
-    if (iu == 1)
-        launch_pdl(k_update32<1>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
-                   cons_next, p4, clocks, runs, (int)n_runs);
-    else if (iu == 2)
-        launch_pdl(k_update32<2>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
-                   cons_next, p4, clocks, runs, (int)n_runs);
-    else
-        launch_pdl(k_update32<4>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
-                   cons_next, p4, clocks, runs, (int)n_runs);
-    if (marks) cudaEventRecord(marks[3], stream);
-    return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
+    PdlQueue q = {stream};
+    return step_f32(mesh, geo, par, moving, launch, prim4, cons, cons_next, cellrec, w2, flux4, clocks, n_runs, cell_run,
+                    q, marks);
 }
 
 int phd_steps_f32(const phd_mesh *mesh, const phd_geom32 *geo, const phd_params *par, int32_t moving,
@@ -1396,10 +1470,11 @@ int phd_steps_f32(const phd_mesh *mesh, const phd_geom32 *geo, const phd_params 
                   float *flux4, phd_clock *clocks, int32_t n_runs, const int32_t *cell_run, int32_t n_steps,
                   cudaStream_t stream) {
     if (n_steps < 0) return PHD_ERR_ARG;
+    PdlQueue q = {stream};
     for (int k = 0; k < n_steps; k++) {
-        const int rc = phd_step_f32_batched(mesh, geo, par, moving, launch, prim4, (k & 1) ? cons_other : cons,
-                                            (k & 1) ? cons : cons_other, cellrec, w2, flux4, clocks, n_runs, cell_run,
-                                            stream, nullptr);
+        phd::NvtxRange nvtx_range("phd_step_f32");
+        const int rc = step_f32(mesh, geo, par, moving, launch, prim4, (k & 1) ? cons_other : cons,
+                                (k & 1) ? cons : cons_other, cellrec, w2, flux4, clocks, n_runs, cell_run, q, nullptr);
         if (rc != PHD_OK) return rc;
     }
     return PHD_OK;
