@@ -1220,6 +1220,10 @@ inline int grid_for(int n, int block, int cap) {
 // a thread where there are several waves of them: 63.5 -> 55.7 us at 3.1M faces, 20.5 -> 18.5
 // at 0.8M.  The exact solver's, long and uneven, takes blocks of one warp (a step at 1M cells 742 ->
 // 668 us, at 0.2M 172 -> 156, against blocks of 256).
+// Meshes of less than a wave take blocks of 64, which spread evenly over the SMs where a few
+// blocks of 256 leave some with twice the work: 13.7 -> 13.0 us a step at 10,000 cells, 18.0 ->
+// 17.4 at 66,000 (HLL and TESS 14.3 -> 13.4, 18.4 -> 18.0, at 41,000 21.3 -> 18.4); at 111,000
+// 22.4 -> 22.7, and below 16 cells an SM nothing is gained (11.4 -> 11.6 at 300 cells).
 inline phd_launch default_launch(const phd_mesh &M, int solver) {
     const int sms = sm_count_current();
     phd_launch L = {256, 128, 256, 0, 0, 0, 1, 1, 1};
@@ -1227,6 +1231,7 @@ inline phd_launch default_launch(const phd_mesh &M, int solver) {
         L.grid_cap_grad = L.grid_cap_update = 4 * sms;
         if (M.n_cells > 2048 * sms) L.block_update = 384;   // up to there two even rounds of 1024 threads
     }
+    if (M.n_cells > 16 * sms && M.n_cells <= 512 * sms) L.block_grad = L.block_face = L.block_update = 64;
     if (solver == PHD_EXACT) L.block_face = 32;
     else if (M.n_faces > 2 * 1280 * sms) L.items_face = 2;
     return L;
