@@ -214,47 +214,66 @@ __device__ __forceinline__ void block_min_to_f(float v, unsigned long long *slot
 
 // Turn one run's CFL minimum into its next time step (cfl * min, clipped to land on
 // t_end) and re-arm its accumulator; with `advance` the clock first moves past the
-// step just taken (t += dt, step += 1).
-__device__ __forceinline__ void finalize_clock(phd_clock *clk, double cfl, bool advance) {
-    const unsigned long long bits = atomicAdd(&clk->dtmin_bits, 0ull);
-    const double mn = __longlong_as_double(static_cast<long long>(bits));
+// step just taken (t += dt, step += 1).  now: the clock's fields as this kernel found them.
+struct ClockNow {
+    double dt, t, t_end;
+    long long step;
+};
+
+__device__ __forceinline__ ClockNow clock_now(const phd_clock *clk) { return {clk->dt, clk->t, clk->t_end, clk->step}; }
+
+__device__ __forceinline__ void finalize_clock(phd_clock *clk, const ClockNow &now, double cfl, bool advance) {
+    const unsigned long long bits = atomicExch(&clk->dtmin_bits, dbits(INFINITY));
+    double t = now.t, dt = cfl * __longlong_as_double(static_cast<long long>(bits));
     if (advance) {
-        clk->t = clk->t + clk->dt;
-        clk->dt_last = clk->dt;
-        clk->step = clk->step + 1;
+        t = t + now.dt;
+        clk->t = t;
+        clk->dt_last = now.dt;
+        clk->step = now.step + 1;
     }
-    double dt = cfl * mn;
     clk->dt_hydro = dt;
     // Time.modify_timestep + Simulation.compute_time_step (simulation_finish.py:82-88,
     // simulation.py:201-212): land exactly on t_end.
-    if (clk->t_end > 0.0 && clk->t + dt >= clk->t_end) dt = fmin(clk->t_end - clk->t, dt);
+    if (now.t_end > 0.0 && t + dt >= now.t_end) dt = fmin(now.t_end - t, dt);
     clk->dt = dt;
-    clk->dtmin_bits = dbits(INFINITY);
 }
 
 // Finish a grid-wide CFL reduction over n_runs clocks: the last block to arrive
 // finalises every run.  No block waits on another: every block reads the clocks'
 // dt before its arrival is counted (clocks[0].arrive), and only the last arrival
 // writes them.  The block's minimum reached L2 through an atomic issued by thread 0
-// (block_min_to / block_min_to_f); thread 0 alone fences before counting the arrival
-// (release), so the block's other threads never wait for their own outstanding stores.
-// Per-run minima issued by other threads (the batched path) are fenced where they are
-// issued (atomic_min_fenced).
+// (block_min_to / block_min_to_f), and the arrival is counted by thread 0 with release and
+// acquire order, so the block's other threads never wait for their own outstanding stores.
+// With one run thread 0 finalises it by itself, the clock's fields loaded ahead: the end of
+// a step is a chain of L2 round trips (minimum, arrival, exchange), two fewer than with the
+// clock read by a whole block between barriers and fences (1,000 cells, FP32: 13.4 -> 12.7 us
+// a step; 10,000 cells, FP64: 67.1 -> 66.1).  Per-run minima issued by
+// other threads (the batched path) are fenced where they are issued (atomic_min_fenced).
+__device__ __forceinline__ unsigned int arrive_acq_rel(unsigned int *p) {
+    unsigned int prev;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(prev) : "l"(__cvta_generic_to_global(p)) : "memory");
+    return prev;
+}
+
 __device__ __forceinline__ void finish_cfl_multi(phd_clock *clocks, int n_runs, double cfl, bool advance) {
+    if (n_runs == 1) {
+        if (threadIdx.x == 0) {
+            const ClockNow now = clock_now(clocks);
+            if (arrive_acq_rel(&clocks[0].arrive) == gridDim.x - 1) {
+                finalize_clock(clocks, now, cfl, advance);
+                clocks[0].arrive = 0u;
+            }
+        }
+        return;
+    }
     __shared__ bool s_last;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned int prev = atomicAdd(&clocks[0].arrive, 1u);
-        s_last = (prev == gridDim.x - 1);
-    }
+    if (threadIdx.x == 0) s_last = arrive_acq_rel(&clocks[0].arrive) == gridDim.x - 1;
     __syncthreads();
     if (s_last) {
         __threadfence();
-        for (int r = threadIdx.x; r < n_runs; r += blockDim.x) finalize_clock(clocks + r, cfl, advance);
-        __syncthreads();
+        for (int r = threadIdx.x; r < n_runs; r += blockDim.x) finalize_clock(clocks + r, clock_now(clocks + r), cfl, advance);
         if (threadIdx.x == 0) clocks[0].arrive = 0u;
-        __threadfence();
     }
 }
 
