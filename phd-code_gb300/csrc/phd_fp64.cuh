@@ -234,6 +234,21 @@ PHD_HD __forceinline__ float f64_to_f32(double a) {
 #endif
 }
 
+// The same of a 2^-e for magnitudes up to 2^20, a NaN above.
+PHD_HD __forceinline__ float f64_to_f32_scaled(double a, int e) {
+    const unsigned long long b = (unsigned long long)f64_bits(a);
+    const int ex = (int)((b >> 52) & 0x7ffu) - 896 - e;
+    const unsigned m = (unsigned)(b >> 29) & 0x7fffffu, s = (unsigned)(b >> 32) & 0x80000000u;
+    const unsigned u = ex <= 0 ? s : (ex >= 147 ? 0x7fc00000u : (s | ((unsigned)ex << 23) | m));
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
+    float f;
+    memcpy(&f, &u, sizeof f);
+    return f;
+#endif
+}
+
 // ---- powers in 64-bit fixed point -----------------------------------------------------
 // x^y = 2^(y log2 x) for positive x by some 400 integer instructions, which run in the shadow
 // of the FP64 pipe (CUDA's pow is 84 FP64 instructions: 1600 clocks a warp and SM, measured).

@@ -72,3 +72,18 @@ def test_gradients_match_oracle(kind, limiter):
     assert np.array_equal(np.repeat(tf[8:12, :nr], 2, axis=0) * tf[:8, :nr], g[:, :nr])
     e = ti[:12, :nr]
     assert np.all((e < 0) | ((e >= mesh.nbr_ptr[:nr]) & (e < mesh.nbr_ptr[1:nr + 1])))
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -300, 1.0, 2.0 ** 200])
+@pytest.mark.parametrize("slope", [(1.0, 1.0), (1.0, -1.0), (1.0, 0.0), (0.0, 0.0), (1.0, 2.0 ** -40)])
+def test_largest_change_among_equals(slope, scale):
+    """The limiter's face where several are equal or nearly so: regular lattices, where the
+    separations repeat up to their rounding, with slopes along the axes and the diagonals."""
+    mesh, _ = pkg.meshgen.build_mesh(pkg.meshgen.jittered_lattice(9, jitter=0.0, seed=1), "reflective")
+    wave = slope[0] * mesh.x[0] + slope[1] * mesh.x[1]
+    bump = np.where((mesh.x[0] > 0.4) & (mesh.x[1] > 0.4), 1.0, 0.0)
+    prim = pkg.meshgen.fill_ghosts(mesh, np.stack([3.0 + wave, wave, bump, 3.0 + bump + wave]) * scale)
+    want, status = O.gradients(mesh, prim, 0)
+    assert status == 0
+    got = device_gradients(mesh, prim, "arepo")
+    assert_parity(got, want)
