@@ -8,7 +8,8 @@
 //                  temporal and spatial stages -> 24 per-face adjoint values
 //   k_adj_cell     per cell: sum its faces' contributions; a real cell with its ghost rows
 //                  folded in, through the reverse of the limited gradient -> per-entry
-//                  neighbour adjoints and the cell's own adjoint
+//                  neighbour adjoints and the cell's own adjoint (k_adj_cell_taped after a taped
+//                  forward step, four threads a cell)
 //   k_adj_final    per real cell: own and ghost rows' sums and the neighbours' parts through
 //                  the reverse of the primitive recovery, lam = lam' + J^T lam_prim
 
@@ -281,19 +282,17 @@ __device__ __forceinline__ void gather_row(const phd_mesh &M, const double *__re
 // prim_part, the neighbours' to entry_adj, the own one added to prim_part.  Ghost rows' entries
 // get zeros (their gradient is their image's).  LINEAR: false for constant reconstruction,
 // which has no gradients.
-// TAPED: the forward selections (unlimited estimate, limiter values, active entries,
-// neighbour extrema) come from the limiter record of a taped forward step instead of
-// being recomputed.
+// The forward selections (unlimited estimate, limiter values, active entries, neighbour
+// extrema) are recomputed here; k_adj_cell_taped reads them from the limiter record of a
+// taped forward step.
 // One kernel where a gather per cell, two clears and this reverse were four launches; the
 // reverse's own arithmetic is fused multiply-adds on a reciprocal per entry (phd_fp64.cuh),
 // 38 FP64 instructions an entry instead of 80.
-template <bool LINEAR, bool TAPED>
+template <bool LINEAR>
 __global__ void __launch_bounds__(128) k_adj_cell(const __grid_constant__ phd_mesh M, phd_adj_index A, int limiter,
                                                   const double *__restrict__ prim, const double *__restrict__ face_adj,
                                                   double *__restrict__ entry_adj /* [4][2F] */,
-                                                  double *__restrict__ prim_part /* [4][n] */,
-                                                  const double *__restrict__ tape_f64,
-                                                  const int32_t *__restrict__ tape_i32) {
+                                                  double *__restrict__ prim_part /* [4][n] */) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= M.n_cells) return;
     const int n = M.n_cells, F = M.n_faces;
@@ -337,69 +336,56 @@ __global__ void __launch_bounds__(128) k_adj_cell(const __grid_constant__ phd_me
         cx[k] = xi[k] + M.dcom[(size_t)k * n + c];
     }
     const double vol = M.vol[c];
-    if (TAPED) {
-#pragma unroll
-        for (int r = 0; r < 8; r++) df[r] = tape_f64[(size_t)r * n + c];
-#pragma unroll
+    // forward recompute (cell_gradient_f64 with selections)
+    double phi_max[4], phi_min[4];
+    for (int f = 0; f < 4; f++) {
+        pc[f] = prim[(size_t)f * n + c];
+        phi_max[f] = phi_min[f] = pc[f];
+        arg_max[f] = arg_min[f] = -1;
+        df[2 * f] = df[2 * f + 1] = 0.0;
+    }
+    for (int e = m0; e < m1; e++) {
+        const int fid = M.nbr_idx[e];
+        const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
+        const double area = M.area[fid];
+        double cfx[2], dr[2], r = 0.0;
+        for (int k = 0; k < 2; k++) {
+            const double xj = M.x[(size_t)k * n + j];
+            cfx[k] = M.com[(size_t)k * F + fid] - 0.5 * (xi[k] + xj);
+            dr[k] = xi[k] - xj;
+            r = r + t_sq(dr[k]);
+        }
+        r = sqrt(r);
         for (int f = 0; f < 4; f++) {
-            alpha[f] = tape_f64[(size_t)(8 + f) * n + c];
-            act[f] = tape_i32[(size_t)f * n + c];
-            arg_max[f] = tape_i32[(size_t)(4 + f) * n + c];
-            arg_min[f] = tape_i32[(size_t)(8 + f) * n + c];
+            const double pj = prim[(size_t)f * n + j];
+            if (pj > phi_max[f]) { phi_max[f] = pj; arg_max[f] = e; }
+            if (pj < phi_min[f]) { phi_min[f] = pj; arg_min[f] = e; }
+            const double d_dif = pj - pc[f], d_sum = pj + pc[f];
+            for (int k = 0; k < 2; k++)
+                df[2 * f + k] = df[2 * f + k] + (area * ((d_dif * cfx[k]) - ((0.5 * d_sum) * dr[k]))) / (r * vol);
         }
-        act_f0 = tape_i32[(size_t)12 * n + c];
-    } else {
-        // forward recompute (cell_gradient_f64 with selections)
-        double phi_max[4], phi_min[4];
+    }
+    for (int e = m0; e < m1; e++) {
+        const int fid = M.nbr_idx[e];
+        const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
+        double sep[2];
+        for (int k = 0; k < 2; k++) sep[k] = M.com[(size_t)k * F + fid] - cx[k];
         for (int f = 0; f < 4; f++) {
-            pc[f] = prim[(size_t)f * n + c];
-            phi_max[f] = phi_min[f] = pc[f];
-            arg_max[f] = arg_min[f] = -1;
-            df[2 * f] = df[2 * f + 1] = 0.0;
-        }
-        for (int e = m0; e < m1; e++) {
-            const int fid = M.nbr_idx[e];
-            const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
-            const double area = M.area[fid];
-            double cfx[2], dr[2], r = 0.0;
-            for (int k = 0; k < 2; k++) {
-                const double xj = M.x[(size_t)k * n + j];
-                cfx[k] = M.com[(size_t)k * F + fid] - 0.5 * (xi[k] + xj);
-                dr[k] = xi[k] - xj;
-                r = r + t_sq(dr[k]);
-            }
-            r = sqrt(r);
-            for (int f = 0; f < 4; f++) {
-                const double pj = prim[(size_t)f * n + j];
-                if (pj > phi_max[f]) { phi_max[f] = pj; arg_max[f] = e; }
-                if (pj < phi_min[f]) { phi_min[f] = pj; arg_min[f] = e; }
-                const double d_dif = pj - pc[f], d_sum = pj + pc[f];
-                for (int k = 0; k < 2; k++)
-                    df[2 * f + k] = df[2 * f + k] + (area * ((d_dif * cfx[k]) - ((0.5 * d_sum) * dr[k]))) / (r * vol);
-            }
-        }
-        for (int e = m0; e < m1; e++) {
-            const int fid = M.nbr_idx[e];
-            const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
-            double sep[2];
-            for (int k = 0; k < 2; k++) sep[k] = M.com[(size_t)k * F + fid] - cx[k];
-            for (int f = 0; f < 4; f++) {
-                double dphi = 0.0, psi;
-                for (int k = 0; k < 2; k++) dphi = dphi + df[2 * f + k] * sep[k];
-                if (limiter == PHD_LIMITER_AREPO) {
-                    if (dphi > 0) psi = (phi_max[f] - pc[f]) / dphi;
-                    else if (dphi < 0) psi = (phi_min[f] - pc[f]) / dphi;
-                    else psi = 1.0;
-                    const double cand = fmax(psi, 0.);
-                    if (cand < alpha[f]) { alpha[f] = cand; act[f] = (psi > 0.0 && dphi != 0.0) ? e : -2; }
-                } else {
-                    if (dphi > 0.0 || dphi < 0.0) {
-                        const double t = (prim[(size_t)f * n + j] - pc[f]) / dphi;
-                        psi = (0. > t) ? 0. : t;
-                    } else psi = 1.0;
-                    const double cand = fmax(psi, 0.);
-                    if (cand < alpha[0]) { alpha[0] = cand; act[0] = (psi > 0.0 && dphi != 0.0) ? e : -2; act_f0 = f; }
-                }
+            double dphi = 0.0, psi;
+            for (int k = 0; k < 2; k++) dphi = dphi + df[2 * f + k] * sep[k];
+            if (limiter == PHD_LIMITER_AREPO) {
+                if (dphi > 0) psi = (phi_max[f] - pc[f]) / dphi;
+                else if (dphi < 0) psi = (phi_min[f] - pc[f]) / dphi;
+                else psi = 1.0;
+                const double cand = fmax(psi, 0.);
+                if (cand < alpha[f]) { alpha[f] = cand; act[f] = (psi > 0.0 && dphi != 0.0) ? e : -2; }
+            } else {
+                if (dphi > 0.0 || dphi < 0.0) {
+                    const double t = (prim[(size_t)f * n + j] - pc[f]) / dphi;
+                    psi = (0. > t) ? 0. : t;
+                } else psi = 1.0;
+                const double cand = fmax(psi, 0.);
+                if (cand < alpha[0]) { alpha[0] = cand; act[0] = (psi > 0.0 && dphi != 0.0) ? e : -2; act_f0 = f; }
             }
         }
     }
@@ -473,6 +459,136 @@ __global__ void __launch_bounds__(128) k_adj_cell(const __grid_constant__ phd_me
     }
 #pragma unroll
     for (int f = 0; f < 4; f++) prim_part[(size_t)f * n + c] = own[f] + aself[f];
+}
+
+// Row x's sums of field f's face contributions (the primitive's, the gradient's two), in list
+// order, the loads of four faces at a time.
+__device__ __forceinline__ void gather_field(const phd_mesh &M, const double *__restrict__ face_adj, int x, int f,
+                                             double &s0, double &s1, double &s2) {
+    const int F = M.n_faces, m0 = M.nbr_ptr[x], m1 = M.nbr_ptr[x + 1];
+    s0 = s1 = s2 = 0.0;
+    constexpr int CH = 4;
+    for (int eb = m0; eb < m1; eb += CH) {
+        int fid[CH];
+        double v[CH][3];
+#pragma unroll
+        for (int k = 0; k < CH; k++) fid[k] = eb + k < m1 ? M.nbr_idx[eb + k] : -1;
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            v[k][0] = v[k][1] = v[k][2] = 0.0;
+            if (fid[k] < 0 || fid[k] >= F) continue;
+            const bool as_i = M.pair_i[fid[k]] == x;
+            const size_t pb = as_i ? 0 : 4, gb = as_i ? 8 : 16;
+            v[k][0] = face_adj[(pb + f) * F + fid[k]];
+            v[k][1] = face_adj[(gb + 2 * f) * F + fid[k]];
+            v[k][2] = face_adj[(gb + 2 * f + 1) * F + fid[k]];
+        }
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            if (fid[k] < 0 || fid[k] >= F) continue;
+            s0 += v[k][0];
+            s1 += v[k][1];
+            s2 += v[k][2];
+        }
+    }
+}
+
+// k_adj_cell<true> after a taped forward step, by four threads a cell, each with one field: the
+// gathered sums and the limiter's reverse are its own, the lists' geometry is formed by one
+// thread an entry and handed round.  A thread a cell left three or four warps on an SM, each
+// with 415 FP64 instructions one behind the other (16,384 cells: 35.4 -> 23.5 us); the sums
+// keep their order.
+__global__ void __launch_bounds__(128) k_adj_cell_taped(const __grid_constant__ phd_mesh M, phd_adj_index A, int limiter,
+                                                        const double *__restrict__ face_adj,
+                                                        double *__restrict__ entry_adj, double *__restrict__ prim_part,
+                                                        const double *__restrict__ tape_f64,
+                                                        const int32_t *__restrict__ tape_i32) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, c = t >> 2, f = t & 3;
+    if (c >= M.n_cells) return;                      // whole quads
+    const unsigned quad = 0xfu << (threadIdx.x & 28);
+    const int n = M.n_cells, F = M.n_faces;
+    const size_t E2 = 2 * (size_t)F;
+    const int m0 = M.nbr_ptr[c], m1 = M.nbr_ptr[c + 1];
+    double own, ag0, ag1;
+    gather_field(M, face_adj, c, f, own, ag0, ag1);
+    if (M.tag[c] != PHD_REAL_TAG) {
+        prim_part[(size_t)f * n + c] = own;          // the primitives' part, folded by k_adj_final
+        for (int e = m0; e < m1; e++) entry_adj[f * E2 + e] = 0.0;
+        return;
+    }
+    for (int g = A.ghost_ptr[c]; g < A.ghost_ptr[c + 1]; g++) {
+        const int x = A.ghost_idx[g], fl = M.flip ? M.flip[x] : 0;
+        double s0, s1, s2;
+        gather_field(M, face_adj, x, f, s0, s1, s2);
+        ag0 += (f == 1 && (fl & 1)) ? -s1 : s1;
+        ag1 += (f == 2 && (fl & 2)) ? -s2 : s2;
+    }
+    const double xc = M.x[c], yc = M.x[(size_t)n + c], cx = xc + M.dcom[c], cy = yc + M.dcom[(size_t)n + c];
+    const double vol = M.vol[c];
+    const double df0 = tape_f64[(size_t)(2 * f) * n + c], df1 = tape_f64[(size_t)(2 * f + 1) * n + c];
+    const double alpha = tape_f64[(size_t)(8 + f) * n + c];
+    const bool tess = limiter == PHD_LIMITER_TESS;
+    // reverse: grad = alpha * df
+    double adf0 = alpha * ag0, adf1 = alpha * ag1, aself = 0.0, aext = 0.0;
+    int ext = -1;                                    // the entry aext belongs to
+    // limiter: active psi -> (extreme value, own value, df); with TESS the density's, whose
+    // entry's ratio is that of field ff
+    double aalpha = fma(df0, ag0, df1 * ag1), al = alpha, d0 = df0, d1 = df1;
+    int act = tape_i32[(size_t)f * n + c], ff = f;
+    if (tess) {
+        act = __shfl_sync(quad, act, 0, 4);
+        ff = act >= 0 ? tape_i32[(size_t)12 * n + c] : 0;
+        aalpha = __shfl_sync(quad, aalpha, 0, 4);
+        al = __shfl_sync(quad, alpha, 0, 4);
+        d0 = __shfl_sync(quad, df0, ff, 4);
+        d1 = __shfl_sync(quad, df1, ff, 4);
+    }
+    if (act >= 0 && ff == f) {
+        const int fid = M.nbr_idx[act];
+        const double s0 = M.com[fid] - cx, s1 = M.com[(size_t)F + fid] - cy;
+        const double dphi = d0 * s0 + d1 * s1;
+        bool ok = true;
+        double y = f64_rcp(dphi, ok);
+        if (!ok) y = 1.0 / dphi;
+        const double ap = aalpha * y, ad = -ap * al;
+        const int arg = tess ? act : tape_i32[(size_t)((f64_pos(dphi) ? 4 : 8) + f) * n + c];
+        adf0 = fma(ad, s0, adf0);
+        adf1 = fma(ad, s1, adf1);
+        if (arg >= 0) {
+            aself -= ap;
+            aext = ap;
+            ext = arg;
+        }
+    }
+    // df = sum_e area (d_dif cfx - d_sum dr / 2) / (r vol)
+    for (int eb = m0; eb < m1; eb += 4) {
+        const int fid = M.nbr_idx[min(eb + f, m1 - 1)];
+        const int j = (M.pair_i[fid] == c) ? M.pair_j[fid] : M.pair_i[fid];
+        const double area = M.area[fid];
+        const double xj = M.x[j], yj = M.x[(size_t)n + j];
+        const double cfx = fma(-0.5, xc + xj, M.com[fid]), cfy = fma(-0.5, yc + yj, M.com[(size_t)F + fid]);
+        const double dx = xc - xj, dy = yc - yj;
+        bool ok = true;
+        double r2 = fma(dx, dx, dy * dy), r = f64_sqrt(r2, ok), y = f64_rcp(r * vol, ok);
+        if (!ok) {
+            r = sqrt(r2);
+            y = 1.0 / (r * vol);
+        }
+        const double coef = area * y;
+        const double jx = coef * fma(-0.5, dx, cfx), jy = coef * fma(-0.5, dy, cfy);      // d df / d phi_j
+        const double sx = -coef * fma(0.5, dx, cfx), sy = -coef * fma(0.5, dy, cfy);      // d df / d phi_c
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (eb + k >= m1) break;                 // uniform over the quad
+            const double Jx = __shfl_sync(quad, jx, k, 4), Jy = __shfl_sync(quad, jy, k, 4);
+            const double Sx = __shfl_sync(quad, sx, k, 4), Sy = __shfl_sync(quad, sy, k, 4);
+            double aj = fma(adf0, Jx, adf1 * Jy);
+            aself = fma(adf0, Sx, fma(adf1, Sy, aself));
+            if (ext == eb + k) aj += aext;
+            entry_adj[f * E2 + eb + k] = aj;
+        }
+    }
+    prim_part[(size_t)f * n + c] = own + aself;
 }
 
 // Per real cell: its rows' primitive adjoints (own and ghosts', flipped) with the neighbours'
@@ -589,16 +705,16 @@ static int adjoint_step(const phd_mesh *mesh, const phd_adj_index *index, const 
     }
     const int bc = block_for((int)n, 128), gc = grid_for_block((int)n, bc);
     if (par->reconstruction != PHD_LINEAR) {
-        k_adj_cell<false, false><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part,
-                                                        nullptr, nullptr);
+        k_adj_cell<false><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part);
         k_adj_final<false><<<gc, bc, 0, stream>>>(M, *index, par->gamma, cons, prim_part, entry_adj, lam_next, lam);
     } else {
-        if (tape_f64)
-            k_adj_cell<true, true><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part,
-                                                          tape_f64, tape_i32);
-        else
-            k_adj_cell<true, false><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part,
-                                                           nullptr, nullptr);
+        if (tape_f64) {
+            const int bt = block_for(4 * (int)n, 128);
+            k_adj_cell_taped<<<grid_for_block(4 * (int)n, bt), bt, 0, stream>>>(M, *index, par->limiter, face_adj, entry_adj,
+                                                                               prim_part, tape_f64, tape_i32);
+        } else {
+            k_adj_cell<true><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part);
+        }
         k_adj_final<true><<<gc, bc, 0, stream>>>(M, *index, par->gamma, cons, prim_part, entry_adj, lam_next, lam);
     }
     return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
