@@ -188,11 +188,17 @@ class FluxRunRecord:
         """lam_n (real cells) from lam_{n+1} at the step's recorded all-cell state
         (cons, prim, grad, tape); with a limiter tape the reverse reads the forward's
         selections instead of recomputing them."""
-        cons, prim, grad, tape = state
         dm = rec.dmesh
         b = self._buffers(dm)
-        lib = L.lib()
         b.lam_next[:, :dm.n_real].copy_(lam_next_real)
+        self._reverse(rec, state, b)
+        return b.lam[:, :dm.n_real].clone()
+
+    def _reverse(self, rec, state, b):
+        """b.lam from b.lam_next (all cells, ghost rows zero in both)."""
+        cons, prim, grad, tape = state
+        dm = rec.dmesh
+        lib = L.lib()
         common = (dm.ref, ctypes.byref(rec.index()), ctypes.byref(self.params), rec.dt, L.ptr(cons), L.ptr(prim),
                   L.ptr(grad), L.ptr(rec.face_w), L.ptr(b.lam_next), L.ptr(b.lam),
                   L.ptr(b.adjoint_work(lib, dm, self.device)))
@@ -201,7 +207,6 @@ class FluxRunRecord:
         else:
             L.check(lib.phd_adjoint_step_f64_taped(*common, L.ptr(tape[0]), L.ptr(tape[1]), L.stream_handle()),
                     "phd_adjoint_step_f64_taped")
-        return b.lam[:, :dm.n_real].clone()
 
     # --- whole run ------------------------------------------------------------------
     def _tail_start(self):
@@ -316,9 +321,11 @@ class FluxRunRecord:
             n = dm.n_cells
             if k > a and self.steps[k - 1].dmesh is not dm:
                 cons, prim = self._loaded(dm, cons[:, :dm.n_real])
-            grad = torch.zeros((8, n), dtype=F64, device=self.device)
             tape = None
-            if self.params.reconstruction == L.LINEAR:
+            if self.params.reconstruction != L.LINEAR:
+                grad = torch.zeros((8, n), dtype=F64, device=self.device)
+            else:
+                grad = torch.empty((8, n), dtype=F64, device=self.device)
                 tape = (torch.empty((L.GRAD_TAPE_F64_ROWS, n), dtype=F64, device=self.device),
                         torch.empty((L.GRAD_TAPE_I32_ROWS, n), dtype=torch.int32, device=self.device))
             states.append((cons, prim, grad, tape))
@@ -337,6 +344,7 @@ class FluxRunRecord:
         """dLoss/dU_0 from dLoss/dU_T, segment by segment (recompute from checkpoints)."""
         lam = lam_T
         N = len(self.steps)
+        prev = None                                     # the buffers whose lam is current
         starts = sorted(self.ckpt)
         for si in range(len(starts) - 1, -1, -1):
             a = starts[si]
@@ -345,9 +353,16 @@ class FluxRunRecord:
             if states is None:
                 states = self._replay_segment(a, b)
             for k in range(b - 1, a - 1, -1):
-                lam = self._adjoint(self.steps[k], states[k - a], lam)
+                rec = self.steps[k]
+                bufs = self._buffers(rec.dmesh)
+                if prev is bufs:                        # the same mesh: lam is the next step's lam_next as it stands
+                    bufs.lam, bufs.lam_next = bufs.lam_next, bufs.lam
+                else:
+                    bufs.lam_next[:, :rec.dmesh.n_real].copy_(lam if prev is None else prev.lam[:, :rec.dmesh.n_real])
+                self._reverse(rec, states[k - a], bufs)
+                prev = bufs
             del states
-        return lam
+        return prev.lam[:, :self.steps[0].dmesh.n_real].clone()
 
 
 def cons_from_prim_t(prim, vol, gamma):
