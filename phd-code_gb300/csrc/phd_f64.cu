@@ -235,6 +235,13 @@ __device__ __noinline__ int gradient_row_plain(const phd_mesh *M, const double *
     return st;
 }
 
+// The step's kernels are launched with programmatic stream serialization (PdlQueue): a kernel's
+// blocks come in as the last ones of the kernel before leave, do what concerns the mesh alone
+// (row setup and lists here, geometry and list heads in the face and update kernels) and wait
+// only then.  Measured against plain launches: 10,000 cells 64 -> 57 us a step, 66,000 240 ->
+// 232, 40 adjoint steps at 128 x 128 9.85 -> 9.5 ms.  Letting them in earlier (launch_dependents on
+// entry) puts most of them on the SMs that happen to be free: 75 us a step at 10,000 cells.
+
 // Limited gradients of NC rows (cells) by 4 NC threads, the same numbers as cell_gradient_f64
 // bit for bit.  The kernel is bound by the FP64 pipe (phd_fp64.cuh), so the work is laid
 // out for few and full FP64 warp instructions:
@@ -357,9 +364,6 @@ __global__ void __launch_bounds__(4 * NC) k_gradients(const __grid_constant__ ph
         S.ptr[tid] = e0;
         S.cell[tid] = len;
     }
-    // a moving step's generator velocities, each row's own
-    if (w && tid >= 3 * NC && c0 + tid - 3 * NC < n)
-        generator_velocity(M, prim, gamma, eta, regularize, c0 + tid - 3 * NC, w);
     __syncthreads();
     static_assert(4 * NC >= 32 + NC, "the second warp holds a thread a row");
     if (tid >= 32 && tid < 32 + NC) {
@@ -430,6 +434,10 @@ __global__ void __launch_bounds__(4 * NC) k_gradients(const __grid_constant__ ph
         }
         if (!ok) S.odd = 1;
     }
+    pdl_wait();                                      // prim: the previous step's update
+    // a moving step's generator velocities, each row's own
+    if (w && tid >= 3 * NC && c0 + tid - 3 * NC < n)
+        generator_velocity(M, prim, gamma, eta, regularize, c0 + tid - 3 * NC, w);
     __syncthreads();
     if (!S.odd) {
         const int n2 = S.ntask[0], nt = n2 + S.ntask[1];
@@ -605,9 +613,9 @@ __device__ __forceinline__ void face_states_f64(const phd_mesh &M, int m, int i,
     }
 }
 
-// The face's geometry and cell values (linear: with the gradients) for the lean states.
-__device__ __forceinline__ void load_face64(const phd_mesh &M, const double *__restrict__ prim,
-                                            const double *__restrict__ grad, int m, int i, int j, bool linear, Face64 &A) {
+// The face's geometry (linear: with the cells' centroids) and its cell values (linear: with the
+// gradients) for the lean states.
+__device__ __forceinline__ void load_geometry64(const phd_mesh &M, int m, int i, int j, bool linear, Face64 &A) {
     const int n = M.n_cells, F = M.n_faces;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
@@ -615,16 +623,22 @@ __device__ __forceinline__ void load_face64(const phd_mesh &M, const double *__r
         A.xj[k] = M.x[(size_t)k * n + j];
         A.com[k] = M.com[(size_t)k * F + m];
     }
-#pragma unroll
-    for (int f = 0; f < 4; f++) { A.pi[f] = prim[(size_t)f * n + i]; A.pj[f] = prim[(size_t)f * n + j]; }
     if (linear) {
-#pragma unroll
-        for (int r = 0; r < 8; r++) { A.gi[r] = grad[(size_t)r * n + i]; A.gj[r] = grad[(size_t)r * n + j]; }
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             A.ci[k] = M.dcom[(size_t)k * n + i];
             A.cj[k] = M.dcom[(size_t)k * n + j];
         }
+    }
+}
+__device__ __forceinline__ void load_values64(const phd_mesh &M, const double *__restrict__ prim,
+                                              const double *__restrict__ grad, int i, int j, bool linear, Face64 &A) {
+    const int n = M.n_cells;
+#pragma unroll
+    for (int f = 0; f < 4; f++) { A.pi[f] = prim[(size_t)f * n + i]; A.pj[f] = prim[(size_t)f * n + j]; }
+    if (linear) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) { A.gi[r] = grad[(size_t)r * n + i]; A.gj[r] = grad[(size_t)r * n + j]; }
     }
 }
 
@@ -661,7 +675,8 @@ __global__ void __launch_bounds__(128) k_states(const __grid_constant__ phd_mesh
     bool ok = false;
     if (!linear || stages == (PHD_STAGE_SPATIAL | PHD_STAGE_TEMPORAL)) {
         Face64 A;
-        load_face64(M, prim, grad, m, i, j, linear, A);
+        load_geometry64(M, m, i, j, linear, A);
+        load_values64(M, prim, grad, i, j, linear, A);
         A.w[0] = face_w ? face_w[m] : 0.0;
         A.w[1] = face_w ? face_w[(size_t)F + m] : 0.0;
         double L[4], R[4];
@@ -774,9 +789,11 @@ __global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ phd_m
     if (i < 0 || i >= n || j < 0 || j >= n) { set_status(clk, PHD_STATUS_BAD_INDEX); return; }
     const bool boost = SOLVER == PHD_EXACT || P.boost != 0;
     const bool linear = P.reconstruction == PHD_LINEAR;
-    const double dt_half = 0.5 * clk->dt;
     Face64 A;
-    load_face64(M, prim, grad, m, i, j, linear, A);
+    load_geometry64(M, m, i, j, linear, A);
+    pdl_wait();                                      // prim, grad, w, the clock: earlier kernels'
+    const double dt_half = 0.5 * clk->dt;
+    load_values64(M, prim, grad, i, j, linear, A);
     bool ok = true;
     if (w) {
         const double wi[2] = {w[i], w[(size_t)n + i]}, wj[2] = {w[j], w[(size_t)n + j]};
@@ -801,6 +818,7 @@ __global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ phd_m
     } else {
         ok = hll64<SOLVER == PHD_HLLC>(L, R, nrm, A.w, C, boost, f) && ok;
     }
+    pdl_launch_dependents();                         // 5% of a step with the exact solver's long last warps
     if (ok) {
         if (w) {
             face_w[m] = A.w[0];
@@ -997,77 +1015,89 @@ __global__ void __launch_bounds__(128) k_update_step(const __grid_constant__ phd
                                                      phd_clock *clk) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = M.n_cells, F = M.n_faces;
-    const double dt = clk->dt;
     const bool boost = (P.solver == PHD_EXACT) ? true : (P.boost != 0);
     double p[4] = {0., 0., 0., 0.}, vol = 0.;
     float c32 = INFINITY;                            // the candidate in FP32; -1: to be formed in any case
+    // the row, its list and the first chunk's faces: the mesh's, loaded ahead of the wait
+    constexpr int CH = 4;
+    int c = -1, m0 = 0, m1 = 0, status = 0, fid[CH], a[CH];
+    double ar[CH];
+    bool real = false;
+    const auto load_faces = [&](int mb) {
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            fid[k] = M.nbr_idx[mb + k < m1 ? mb + k : m0];
+            if (fid[k] < 0 || fid[k] >= F) fid[k] = -1;
+        }
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            const int f = fid[k] < 0 ? 0 : fid[k];
+            a[k] = M.pair_i[f];
+            ar[k] = M.area[f];
+        }
+    };
     if (i < n) {
-        const bool real = M.tag[i] == PHD_REAL_TAG;
-        const int c = real ? i : M.map[i];
+        real = M.tag[i] == PHD_REAL_TAG;
+        c = real ? i : M.map[i];
         if (c >= 0 && c < n) {
-            double U[4];
-            int status = 0;
-#pragma unroll
-            for (int q = 0; q < 4; q++) U[q] = cons[(size_t)q * n + c];
-            const int m0 = M.nbr_ptr[c];
-            int m1 = M.nbr_ptr[c + 1];
-            if (F <= 0 && m1 > m0) { status |= PHD_STATUS_BAD_INDEX; m1 = m0; }
-            constexpr int CH = 4;
-            for (int mb = m0; mb < m1; mb += CH) {
-                int fid[CH], a[CH];
-                double ar[CH], fl[CH][4];
-#pragma unroll
-                for (int k = 0; k < CH; k++) {
-                    fid[k] = M.nbr_idx[mb + k < m1 ? mb + k : m0];
-                    if (fid[k] < 0 || fid[k] >= F) fid[k] = -1;
-                }
-#pragma unroll
-                for (int k = 0; k < CH; k++) {
-                    const int f = fid[k] < 0 ? 0 : fid[k];
-                    a[k] = M.pair_i[f];
-                    ar[k] = M.area[f];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) fl[k][q] = flux[(size_t)q * F + f];
-                }
-#pragma unroll
-                for (int k = 0; k < CH; k++) {
-                    if (mb + k >= m1) break;
-                    if (fid[k] < 0) { status |= PHD_STATUS_BAD_INDEX; continue; }
-                    const double da = dt * ar[k];
-                    const long long sg = a[k] == c ? (long long)0x8000000000000000ull : 0ll;
-#pragma unroll
-                    for (int q = 0; q < 4; q++) U[q] = U[q] + f64_from(f64_bits(da * fl[k][q]) ^ sg);
-                    if (f64_le0(U[0])) status |= PHD_STATUS_NEG_MASS;
-                    if (f64_le0(U[3])) status |= PHD_STATUS_NEG_ENERGY;
-                }
-            }
-            set_status(clk, status);
-            if (!real) {
-                const int fl = M.flip ? M.flip[i] : 0;
-                if (fl & 1) U[1] = -U[1];
-                if (fl & 2) U[2] = -U[2];
-            }
+            m0 = M.nbr_ptr[c];
+            m1 = M.nbr_ptr[c + 1];
             vol = M.vol[i];
-            prim_lean(U, vol, P.gamma, p);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                cons_next[(size_t)q * n + i] = U[q];
-                prim[(size_t)q * n + i] = p[q];
-            }
-            if (real) {
-                // R/c within a few FP32 roundings while the operands are well inside FP32's range
-                const unsigned lo = (1023u - 100u) << 20, span = 200u << 20;
-                const bool in = f64_hi(p[0]) - lo < span && f64_hi(p[3]) - lo < span && f64_hi(vol) - lo < span;
-                const float cs = sqrtf((float)P.gamma * f64_to_f32(p[3]) / f64_to_f32(p[0]));
-                const float vx = f64_to_f32(p[1]), vy = f64_to_f32(p[2]);
-                const float den = boost ? cs : cs + sqrtf(vx * vx + vy * vy);
-                c32 = in ? sqrtf(f64_to_f32(vol) * 0.3183098861837907f) / den : -1.f;
-                if (!(c32 < INFINITY && c32 > 0.f)) c32 = -1.f;
-            }
+            if (F <= 0 && m1 > m0) { status |= PHD_STATUS_BAD_INDEX; m1 = m0; }
+            if (m0 < m1) load_faces(m0);
         } else {
-            set_status(clk, PHD_STATUS_BAD_INDEX);
+            c = -1;
+            status |= PHD_STATUS_BAD_INDEX;
         }
     }
+    pdl_wait();                                      // flux: the face kernel's; cons, the clock
+    if (c >= 0) {
+        const double dt = clk->dt;
+        double U[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) U[q] = cons[(size_t)q * n + c];
+        for (int mb = m0; mb < m1; mb += CH) {
+            if (mb != m0) load_faces(mb);
+            double fl[CH][4];
+#pragma unroll
+            for (int k = 0; k < CH; k++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) fl[k][q] = flux[(size_t)q * F + (fid[k] < 0 ? 0 : fid[k])];
+#pragma unroll
+            for (int k = 0; k < CH; k++) {
+                if (mb + k >= m1) break;
+                if (fid[k] < 0) { status |= PHD_STATUS_BAD_INDEX; continue; }
+                const double da = dt * ar[k];
+                const long long sg = a[k] == c ? (long long)0x8000000000000000ull : 0ll;
+#pragma unroll
+                for (int q = 0; q < 4; q++) U[q] = U[q] + f64_from(f64_bits(da * fl[k][q]) ^ sg);
+                if (f64_le0(U[0])) status |= PHD_STATUS_NEG_MASS;
+                if (f64_le0(U[3])) status |= PHD_STATUS_NEG_ENERGY;
+            }
+        }
+        if (!real) {
+            const int fl = M.flip ? M.flip[i] : 0;
+            if (fl & 1) U[1] = -U[1];
+            if (fl & 2) U[2] = -U[2];
+        }
+        prim_lean(U, vol, P.gamma, p);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            cons_next[(size_t)q * n + i] = U[q];
+            prim[(size_t)q * n + i] = p[q];
+        }
+        if (real) {
+            // R/c within a few FP32 roundings while the operands are well inside FP32's range
+            const unsigned lo = (1023u - 100u) << 20, span = 200u << 20;
+            const bool in = f64_hi(p[0]) - lo < span && f64_hi(p[3]) - lo < span && f64_hi(vol) - lo < span;
+            const float cs = sqrtf((float)P.gamma * f64_to_f32(p[3]) / f64_to_f32(p[0]));
+            const float vx = f64_to_f32(p[1]), vy = f64_to_f32(p[2]);
+            const float den = boost ? cs : cs + sqrtf(vx * vx + vy * vy);
+            c32 = in ? sqrtf(f64_to_f32(vol) * 0.3183098861837907f) / den : -1.f;
+            if (!(c32 < INFINITY && c32 > 0.f)) c32 = -1.f;
+        }
+    }
+    set_status(clk, status);
     __shared__ float s_c32[4];
     const float wmin = warp_min_f(c32 < 0.f ? INFINITY : c32);
     if ((threadIdx.x & 31) == 0) s_c32[threadIdx.x >> 5] = wmin;
@@ -1085,6 +1115,7 @@ __global__ void __launch_bounds__(128) k_update_step(const __grid_constant__ phd
 // and the steps without gradients.
 __global__ void __launch_bounds__(BLOCK) k_gen_vel(const __grid_constant__ phd_mesh M, const double *__restrict__ prim,
                                                    double gamma, double eta, int regularize, double *__restrict__ w) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < M.n_cells) generator_velocity(M, prim, gamma, eta, regularize, i, w);
 }
@@ -1112,38 +1143,38 @@ inline int grid_of(int n) { return grid_for_block(n, blk_of(n)); }
 // eight steps at 10,000 cells, 4.13 against 4.16 ms for one at a million); w: with a moving step's generator
 // velocities (par's eta and regularize).
 inline void launch_gradients(const phd_mesh &M, const double *prim, int limiter, double *grad, phd_clock *clk,
-                             GradTape tape, double *w, const phd_params *par, cudaStream_t stream) {
+                             GradTape tape, double *w, const phd_params *par, PdlQueue &queue) {
     constexpr int NC = 16;
     const int grid = (M.n_cells + NC - 1) / NC;
     const double gamma = par ? par->gamma : 0., eta = par ? par->eta : 0.;
     const int reg = par ? par->regularize : 0;
     if (tape.f64)
-        k_gradients<NC, true><<<grid, 4 * NC, 0, stream>>>(M, prim, limiter, grad, clk, tape, w, gamma, eta, reg);
+        launch_pdl(k_gradients<NC, true>, grid, 4 * NC, queue, M, prim, limiter, grad, clk, tape, w, gamma, eta, reg);
     else
-        k_gradients<NC, false><<<grid, 4 * NC, 0, stream>>>(M, prim, limiter, grad, clk, tape, w, gamma, eta, reg);
+        launch_pdl(k_gradients<NC, false>, grid, 4 * NC, queue, M, prim, limiter, grad, clk, tape, w, gamma, eta, reg);
 }
 
 inline void launch_gen_vel(const phd_mesh &M, const double *prim, double gamma, double eta, int regularize, double *w,
-                           cudaStream_t stream) {
+                           PdlQueue &queue) {
     const int block = block_for(M.n_cells, BLOCK);
-    k_gen_vel<<<grid_for_block(M.n_cells, block), block, 0, stream>>>(M, prim, gamma, eta, regularize, w);
+    launch_pdl(k_gen_vel, grid_for_block(M.n_cells, block), block, queue, M, prim, gamma, eta, regularize, w);
 }
 
 // Face fluxes; w: the generator velocities of a moving step, from which face_w is formed,
 // or null (face_w as given).
 inline void launch_face_flux(const phd_mesh &M, const phd_params &P, const double *prim, const double *grad,
-                             const double *w, double *face_w, double *flux, phd_clock *clk, cudaStream_t stream) {
+                             const double *w, double *face_w, double *flux, phd_clock *clk, PdlQueue &queue) {
     // one warp a block while there are fewer than 16 an SM: the pipe's work is then spread to
     // a warp's grain
     const int block = M.n_faces < 16 * 128 * sm_count_current() ? 32 : 128, grid = grid_for_block(M.n_faces, block);
     const Gas64 C = gas64(P.gamma);
     const Exact64 X = exact64(P.gamma);
     if (P.solver == PHD_HLL)
-        k_face_flux<PHD_HLL><<<grid, block, 0, stream>>>(M, P, C, X, prim, grad, w, face_w, flux, clk);
+        launch_pdl(k_face_flux<PHD_HLL>, grid, block, queue, M, P, C, X, prim, grad, w, face_w, flux, clk);
     else if (P.solver == PHD_HLLC)
-        k_face_flux<PHD_HLLC><<<grid, block, 0, stream>>>(M, P, C, X, prim, grad, w, face_w, flux, clk);
+        launch_pdl(k_face_flux<PHD_HLLC>, grid, block, queue, M, P, C, X, prim, grad, w, face_w, flux, clk);
     else
-        k_face_flux<PHD_EXACT><<<grid, block, 0, stream>>>(M, P, C, X, prim, grad, w, face_w, flux, clk);
+        launch_pdl(k_face_flux<PHD_EXACT>, grid, block, queue, M, P, C, X, prim, grad, w, face_w, flux, clk);
 }
 
 inline int launch_status() {
@@ -1177,14 +1208,16 @@ const char *phd_status_string(int bit) {
 int phd_gradients_f64(const phd_mesh *mesh, const double *prim, int32_t limiter, double *grad,
                       phd_clock *clk, cudaStream_t stream) {
     if (!mesh_ok(mesh) || !prim || !grad) return PHD_ERR_ARG;
-    launch_gradients(*mesh, prim, limiter, grad, clk, GradTape{nullptr, nullptr}, nullptr, nullptr, stream);
+    PdlQueue queue = {stream};
+    launch_gradients(*mesh, prim, limiter, grad, clk, GradTape{nullptr, nullptr}, nullptr, nullptr, queue);
     return launch_status();
 }
 
 int phd_gradients_f64_taped(const phd_mesh *mesh, const double *prim, int32_t limiter, double *grad,
                             double *tape_f64, int32_t *tape_i32, phd_clock *clk, cudaStream_t stream) {
     if (!mesh_ok(mesh) || !prim || !grad || !tape_f64 || !tape_i32) return PHD_ERR_ARG;
-    launch_gradients(*mesh, prim, limiter, grad, clk, GradTape{tape_f64, tape_i32}, nullptr, nullptr, stream);
+    PdlQueue queue = {stream};
+    launch_gradients(*mesh, prim, limiter, grad, clk, GradTape{tape_f64, tape_i32}, nullptr, nullptr, queue);
     return launch_status();
 }
 
@@ -1258,7 +1291,8 @@ int phd_time_step_f64(const phd_mesh *mesh, const double *prim, double gamma, do
 int phd_generator_velocities_f64(const phd_mesh *mesh, const double *prim, double gamma, double eta,
                                  int32_t regularize, double *w, cudaStream_t stream) {
     if (!mesh_ok(mesh) || !prim || !w) return PHD_ERR_ARG;
-    launch_gen_vel(*mesh, prim, gamma, eta, regularize, w, stream);
+    PdlQueue queue = {stream};
+    launch_gen_vel(*mesh, prim, gamma, eta, regularize, w, queue);
     return launch_status();
 }
 
@@ -1271,13 +1305,14 @@ int phd_face_velocities_f64(const phd_mesh *mesh, const double *w, double *face_
 
 static int step_f64(const phd_mesh *mesh, const phd_params *par, int32_t moving, double *prim, const double *cons,
                     double *cons_next, double *grad, double *w, double *face_w, double *flux, phd_clock *clk,
-                    cudaStream_t stream, cudaEvent_t *marks, GradTape tape);
+                    PdlQueue &queue, cudaEvent_t *marks, GradTape tape);
 
 int phd_step_f64_marked(const phd_mesh *mesh, const phd_params *par, int32_t moving, double *prim,
                         const double *cons, double *cons_next, double *grad, double *w, double *face_w,
                         double *flux, phd_clock *clk, cudaStream_t stream, cudaEvent_t *marks) {
     phd::NvtxRange nvtx_range("phd_step_f64");
-    return step_f64(mesh, par, moving, prim, cons, cons_next, grad, w, face_w, flux, clk, stream, marks,
+    PdlQueue queue = {stream};
+    return step_f64(mesh, par, moving, prim, cons, cons_next, grad, w, face_w, flux, clk, queue, marks,
                     GradTape{nullptr, nullptr});
 }
 
@@ -1286,30 +1321,31 @@ int phd_step_f64_taped(const phd_mesh *mesh, const phd_params *par, int32_t movi
                        double *flux, double *tape_f64, int32_t *tape_i32, phd_clock *clk, cudaStream_t stream) {
     phd::NvtxRange nvtx_range("phd_step_f64_taped");
     if (!tape_f64 || !tape_i32) return PHD_ERR_ARG;
-    return step_f64(mesh, par, moving, prim, cons, cons_next, grad, w, face_w, flux, clk, stream, nullptr,
+    PdlQueue queue = {stream};
+    return step_f64(mesh, par, moving, prim, cons, cons_next, grad, w, face_w, flux, clk, queue, nullptr,
                     GradTape{tape_f64, tape_i32});
 }
 
 static int step_f64(const phd_mesh *mesh, const phd_params *par, int32_t moving, double *prim, const double *cons,
                     double *cons_next, double *grad, double *w, double *face_w, double *flux, phd_clock *clk,
-                    cudaStream_t stream, cudaEvent_t *marks, GradTape tape) {
+                    PdlQueue &queue, cudaEvent_t *marks, GradTape tape) {
     if (!mesh_ok(mesh) || !par || !prim || !cons || !cons_next || !flux || !clk) return PHD_ERR_ARG;
     if (mesh->n_faces && !mesh->normal) return PHD_ERR_ARG;
     const bool linear = par->reconstruction == PHD_LINEAR;
     if (linear && !grad) return PHD_ERR_ARG;
     if (moving && (!w || !face_w)) return PHD_ERR_ARG;
-    if (marks) cudaEventRecord(marks[0], stream);
+    if (marks) cudaEventRecord(marks[0], queue.stream);
     if (linear)
-        launch_gradients(*mesh, prim, par->limiter, grad, clk, tape, moving ? w : nullptr, par, stream);
+        launch_gradients(*mesh, prim, par->limiter, grad, clk, tape, moving ? w : nullptr, par, queue);
     else if (moving)
-        launch_gen_vel(*mesh, prim, par->gamma, par->eta, par->regularize, w, stream);
-    if (marks) cudaEventRecord(marks[1], stream);
+        launch_gen_vel(*mesh, prim, par->gamma, par->eta, par->regularize, w, queue);
+    if (marks) cudaEventRecord(marks[1], queue.stream);
     if (mesh->n_faces)
-        launch_face_flux(*mesh, *par, prim, grad, moving ? w : nullptr, face_w, flux, clk, stream);
-    if (marks) cudaEventRecord(marks[2], stream);
+        launch_face_flux(*mesh, *par, prim, grad, moving ? w : nullptr, face_w, flux, clk, queue);
+    if (marks) cudaEventRecord(marks[2], queue.stream);
     const int bc = block_for(mesh->n_cells, 128);
-    k_update_step<<<grid_for_block(mesh->n_cells, bc), bc, 0, stream>>>(*mesh, *par, flux, cons, cons_next, prim, clk);
-    if (marks) cudaEventRecord(marks[3], stream);
+    launch_pdl(k_update_step, grid_for_block(mesh->n_cells, bc), bc, queue, *mesh, *par, (const double *)flux, cons, cons_next, prim, clk);
+    if (marks) cudaEventRecord(marks[3], queue.stream);
     return launch_status();
 }
 
@@ -1325,9 +1361,11 @@ int phd_steps_f64(const phd_mesh *mesh, const phd_params *par, int32_t moving, d
                   double *cons_other, double *grad, double *w, double *face_w, double *flux, phd_clock *clk,
                   int32_t n_steps, cudaStream_t stream) {
     if (n_steps < 0) return PHD_ERR_ARG;
+    PdlQueue queue = {stream};
     for (int k = 0; k < n_steps; k++) {
-        const int rc = phd_step_f64(mesh, par, moving, prim, (k & 1) ? cons_other : cons, (k & 1) ? cons : cons_other, grad,
-                                    w, face_w, flux, clk, stream);
+        phd::NvtxRange nvtx_range("phd_step_f64");
+        const int rc = step_f64(mesh, par, moving, prim, (k & 1) ? cons_other : cons, (k & 1) ? cons : cons_other, grad, w,
+                                face_w, flux, clk, queue, nullptr, GradTape{nullptr, nullptr});
         if (rc != PHD_OK) return rc;
     }
     return PHD_OK;
