@@ -289,7 +289,8 @@ __device__ __forceinline__ float4 entry_t_of(const EntrySrc &S, int e) {
 // dependent loads of a list pass while that one drains; the face and update kernels do the
 // same with their mesh rows.  On a mesh that is one wave of blocks or less the step is a
 // chain of such latencies: 15.4 -> 13.1 us at 1,000 cells, 28.2 -> 25.4 at 111,000 (HLL,
-// TESS).  Threads that loop load in place: they hide the latency behind each other, and the
+// TESS); with the next kernel's blocks let in as the last ones leave, not on entry (they then
+// sat on the SMs that happened to be free), 11.7 and 23.0.  Threads that loop load in place: they hide the latency behind each other, and the
 // rows kept across the wait cost registers (the update's 58 against 40).  (Loading the next
 // cell's rows during the current one measured about 1 us slower for the same reason.)
 template <bool REC>
@@ -500,7 +501,6 @@ __global__ void __launch_bounds__(512) k_grad32(phd_mesh M, phd_params P, int mo
                                                 const float4 *__restrict__ cell_geo,
                                                 const float4 *__restrict__ prim4, float4 *__restrict__ cellrec,
                                                 float2 *__restrict__ w2, phd_clock *clk) {
-    pdl_launch_dependents();
     if (ITEMS == 0) {
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
         GradHead<REC> H = grad_head<REC, true>(i, M, S, csr_nbr, cell_geo);
@@ -841,7 +841,6 @@ __global__ void __launch_bounds__(FACE_MAX_BLOCK, SOLVER == PHD_EXACT ? 1 : 5) k
                                                 const float4 *__restrict__ cellrec, const float2 *__restrict__ w2,
                                                 float4 *__restrict__ flux4, phd_clock *clocks,
                                                 const int32_t *__restrict__ cell_run, const __grid_constant__ GasC GC) {
-    pdl_launch_dependents();
     if (ITEMS == 0) {
         const int m = blockIdx.x * blockDim.x + threadIdx.x;
         const FaceHead H = face_head(m, M, face_geo, face_ar);
@@ -992,7 +991,6 @@ __global__ void __launch_bounds__(512) k_update32(phd_mesh M, phd_params P, cons
                                                   const double *__restrict__ cons, double *__restrict__ cons_next,
                                                   float4 *__restrict__ prim4, phd_clock *clocks,
                                                   const int32_t *__restrict__ cell_run, int n_runs) {
-    pdl_launch_dependents();
     const int n = M.n_cells;
     const float gam = narrow_f64(P.gamma);
     constexpr int K = ITEMS == 0 ? 1 : ITEMS;
@@ -1030,6 +1028,7 @@ __global__ void __launch_bounds__(512) k_update32(phd_mesh M, phd_params P, cons
             }
         }
     }
+    pdl_launch_dependents();                          // the next step's blocks come in while the clock is advanced
     if (!cell_run) block_min_to_f(cand_all, &clocks[0].dtmin_bits);
     finish_cfl_multi(clocks, cell_run ? n_runs : 1, P.cfl, true);
 }
