@@ -295,6 +295,7 @@ __global__ void __launch_bounds__(128) k_adj_cell(const __grid_constant__ phd_me
                                                   double *__restrict__ prim_part /* [4][n] */) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= M.n_cells) return;
+    pdl_wait();                                      // face_adj: the face kernel's
     const int n = M.n_cells, F = M.n_faces;
     const size_t E2 = 2 * (size_t)F;
     const int m0 = M.nbr_ptr[c], m1 = M.nbr_ptr[c + 1];
@@ -509,9 +510,16 @@ __global__ void __launch_bounds__(128) k_adj_cell_taped(const __grid_constant__ 
     const int n = M.n_cells, F = M.n_faces;
     const size_t E2 = 2 * (size_t)F;
     const int m0 = M.nbr_ptr[c], m1 = M.nbr_ptr[c + 1];
+    const bool real = M.tag[c] == PHD_REAL_TAG;
+    const double xc = M.x[c], yc = M.x[(size_t)n + c], cx = xc + M.dcom[c], cy = yc + M.dcom[(size_t)n + c];
+    const double vol = M.vol[c];
+    const double df0 = tape_f64[(size_t)(2 * f) * n + c], df1 = tape_f64[(size_t)(2 * f + 1) * n + c];
+    const double alpha = tape_f64[(size_t)(8 + f) * n + c];
+    int act = tape_i32[(size_t)f * n + c], ff = f;
+    pdl_wait();                                      // face_adj: the face kernel's
     double own, ag0, ag1;
     gather_field(M, face_adj, c, f, own, ag0, ag1);
-    if (M.tag[c] != PHD_REAL_TAG) {
+    if (!real) {
         prim_part[(size_t)f * n + c] = own;          // the primitives' part, folded by k_adj_final
         for (int e = m0; e < m1; e++) entry_adj[f * E2 + e] = 0.0;
         return;
@@ -523,10 +531,6 @@ __global__ void __launch_bounds__(128) k_adj_cell_taped(const __grid_constant__ 
         ag0 += (f == 1 && (fl & 1)) ? -s1 : s1;
         ag1 += (f == 2 && (fl & 2)) ? -s2 : s2;
     }
-    const double xc = M.x[c], yc = M.x[(size_t)n + c], cx = xc + M.dcom[c], cy = yc + M.dcom[(size_t)n + c];
-    const double vol = M.vol[c];
-    const double df0 = tape_f64[(size_t)(2 * f) * n + c], df1 = tape_f64[(size_t)(2 * f + 1) * n + c];
-    const double alpha = tape_f64[(size_t)(8 + f) * n + c];
     const bool tess = limiter == PHD_LIMITER_TESS;
     // reverse: grad = alpha * df
     double adf0 = alpha * ag0, adf1 = alpha * ag1, aself = 0.0, aext = 0.0;
@@ -534,7 +538,6 @@ __global__ void __launch_bounds__(128) k_adj_cell_taped(const __grid_constant__ 
     // limiter: active psi -> (extreme value, own value, df); with TESS the density's, whose
     // entry's ratio is that of field ff
     double aalpha = fma(df0, ag0, df1 * ag1), al = alpha, d0 = df0, d1 = df1;
-    int act = tape_i32[(size_t)f * n + c], ff = f;
     if (tess) {
         act = __shfl_sync(quad, act, 0, 4);
         ff = act >= 0 ? tape_i32[(size_t)12 * n + c] : 0;
@@ -609,6 +612,8 @@ __global__ void __launch_bounds__(128) k_adj_final(const __grid_constant__ phd_m
     }
     double ap[4] = {0., 0., 0., 0.};
     const int t0 = A.ghost_ptr[c], t1 = A.ghost_ptr[c + 1];
+    const double m = cons[c], mx = cons[(size_t)n + c], my = cons[2 * (size_t)n + c], vol = M.vol[c];
+    pdl_wait();                                      // prim_part, entry_adj: the cell kernel's
     for (int t = t0 - 1; t < t1; t++) {              // the cell itself, then its ghosts
         const int x = t < t0 ? c : A.ghost_idx[t];
         const int fl = (t >= t0 && M.flip) ? M.flip[x] : 0;
@@ -628,8 +633,6 @@ __global__ void __launch_bounds__(128) k_adj_final(const __grid_constant__ phd_m
 #pragma unroll
         for (int f = 0; f < 4; f++) ap[f] += s[f];
     }
-    const double m = cons[c], mx = cons[(size_t)n + c], my = cons[2 * (size_t)n + c];
-    const double vol = M.vol[c];
     bool ok = true;
     double im = f64_rcp(m, ok), iv = f64_rcp(vol, ok);
     if (!ok) {
@@ -693,29 +696,31 @@ static int adjoint_step(const phd_mesh *mesh, const phd_adj_index *index, const 
     double *face_adj = work;                       // [24][F]
     double *entry_adj = face_adj + 24 * F;         // [4][2F]
     double *prim_part = entry_adj + 8 * F;         // [4][n]
+    // the first kernel waits for the stream, the others come in behind each other
+    PdlQueue queue = {stream};
     if (F && par->solver == PHD_EXACT)
-        k_adj_face_exact<<<ga((int)F), ba((int)F), 0, stream>>>(M, *par, dt, prim, grad, face_w, lam_next, face_adj);
+        launch_pdl(k_adj_face_exact, ga((int)F), ba((int)F), queue, M, *par, dt, prim, grad, face_w, lam_next, face_adj);
     else if (F) {
         const int block = (int)F < 16 * 128 * sm_count_current() ? 32 : 128, grid = grid_for_block((int)F, block);
         const Gas64 C = gas64(par->gamma);
         if (par->solver == PHD_HLLC)
-            k_adj_face<true><<<grid, block, 0, stream>>>(M, *par, C, dt, prim, grad, face_w, lam_next, face_adj);
+            launch_pdl(k_adj_face<true>, grid, block, queue, M, *par, C, dt, prim, grad, face_w, lam_next, face_adj);
         else
-            k_adj_face<false><<<grid, block, 0, stream>>>(M, *par, C, dt, prim, grad, face_w, lam_next, face_adj);
+            launch_pdl(k_adj_face<false>, grid, block, queue, M, *par, C, dt, prim, grad, face_w, lam_next, face_adj);
     }
     const int bc = block_for((int)n, 128), gc = grid_for_block((int)n, bc);
     if (par->reconstruction != PHD_LINEAR) {
-        k_adj_cell<false><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part);
-        k_adj_final<false><<<gc, bc, 0, stream>>>(M, *index, par->gamma, cons, prim_part, entry_adj, lam_next, lam);
+        launch_pdl(k_adj_cell<false>, gc, bc, queue, M, *index, par->limiter, prim, face_adj, entry_adj, prim_part);
+        launch_pdl(k_adj_final<false>, gc, bc, queue, M, *index, par->gamma, cons, prim_part, entry_adj, lam_next, lam);
     } else {
         if (tape_f64) {
             const int bt = block_for(4 * (int)n, 128);
-            k_adj_cell_taped<<<grid_for_block(4 * (int)n, bt), bt, 0, stream>>>(M, *index, par->limiter, face_adj, entry_adj,
-                                                                               prim_part, tape_f64, tape_i32);
+            launch_pdl(k_adj_cell_taped, grid_for_block(4 * (int)n, bt), bt, queue, M, *index, par->limiter, face_adj,
+                       entry_adj, prim_part, tape_f64, tape_i32);
         } else {
-            k_adj_cell<true><<<gc, bc, 0, stream>>>(M, *index, par->limiter, prim, face_adj, entry_adj, prim_part);
+            launch_pdl(k_adj_cell<true>, gc, bc, queue, M, *index, par->limiter, prim, face_adj, entry_adj, prim_part);
         }
-        k_adj_final<true><<<gc, bc, 0, stream>>>(M, *index, par->gamma, cons, prim_part, entry_adj, lam_next, lam);
+        launch_pdl(k_adj_final<true>, gc, bc, queue, M, *index, par->gamma, cons, prim_part, entry_adj, lam_next, lam);
     }
     return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
 }
