@@ -340,7 +340,7 @@ __device__ __forceinline__ void gradient_changes(const GradShared<NC> &S, int k0
 }
 
 template <int NC, bool TAPE>
-__global__ void __launch_bounds__(4 * NC) k_gradients(const __grid_constant__ phd_mesh M, const double *__restrict__ prim, int limiter,
+__global__ void __launch_bounds__(4 * NC, 5) k_gradients(const __grid_constant__ phd_mesh M, const double *__restrict__ prim, int limiter,
                                                       double *__restrict__ grad, phd_clock *clk, GradTape tape,
                                                       double *__restrict__ w, double gamma, double eta, int regularize) {
     __shared__ GradShared<NC> S;
@@ -1139,12 +1139,13 @@ __global__ void __launch_bounds__(BLOCK) k_face_vel(phd_mesh M, const double *__
 inline int blk_of(int n) { return block_for(n, BLOCK); }
 inline int grid_of(int n) { return grid_for_block(n, blk_of(n)); }
 
-// Gradients of n rows: blocks of 16 rows (64 threads: 622 us against 632 with 32 rows for
-// eight steps at 10,000 cells, 4.13 against 4.16 ms for one at a million); w: with a moving step's generator
-// velocities (par's eta and regularize).
+// Gradients of n rows: blocks of 32 rows and 96 registers, 20 warps an SM (against blocks of 16
+// rows at 112 registers, 18 warps: a step of 1024 x 1024 cells 3.19 -> 3.04 ms, of 333 x 333 382 ->
+// 356 us; equal below 20,000 cells); w: with a moving step's generator velocities (par's eta
+// and regularize).
 inline void launch_gradients(const phd_mesh &M, const double *prim, int limiter, double *grad, phd_clock *clk,
                              GradTape tape, double *w, const phd_params *par, PdlQueue &queue) {
-    constexpr int NC = 16;
+    constexpr int NC = 32;
     const int grid = (M.n_cells + NC - 1) / NC;
     const double gamma = par ? par->gamma : 0., eta = par ? par->eta : 0.;
     const int reg = par ? par->regularize : 0;
