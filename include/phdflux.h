@@ -444,8 +444,9 @@ typedef struct phd_launch {
 /* Batched step: n_runs independent runs concatenated into one mesh (disjoint cell and
  * face ranges; ghosts map inside their run) advance together, one launch per stage.
  * clocks[n_runs] holds each run's dt / t / CFL accumulator; cell_run[n_cells] the run
- * of each cell (may be NULL when n_runs == 1).  launch may be NULL (defaults).  Status
- * bits of a run go to clocks[run] (index errors of the gradient stage to clocks[0]). */
+ * of each cell (may be NULL when n_runs == 1).  launch may be NULL (defaults by the mesh's
+ * size).  Status bits of a run go to clocks[run] (index errors of the gradient stage to
+ * clocks[0]). */
 int phd_step_f32_batched(const phd_mesh *mesh, const phd_geom32 *geo, const phd_params *par,
                          int32_t moving, const phd_launch *launch, float *prim4,
                          const double *cons, double *cons_next, float *cellrec, float *w2,
