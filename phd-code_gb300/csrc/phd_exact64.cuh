@@ -6,7 +6,7 @@
 // of the last place where the library's are within 2.  A pressure function and its derivative
 // take one logarithm between them, the powers at p* serve the sampled state too, and the
 // right side is sampled as the mirrored left one.  Twenty library powers a warp made up most of
-// the 2263 FP64 instructions of the face kernel; 360 are left, and 962 -> 265 us at 197,000
+// the 2263 FP64 instructions of the face kernel; 340 are left, and 962 -> 209 us at 197,000
 // faces (point explosion).  A face outside the helpers' windows (vacuum,
 // non-finite states) returns false and takes the plain path.
 #pragma once

@@ -262,7 +262,8 @@ __device__ __noinline__ int gradient_row_plain(const phd_mesh *M, const double *
 //    no faster: 3.23 ms.)
 // A block that meets anything unusual -- an index out of range, a cell that its face does not
 // name, more list entries than the shared arrays hold, an operand outside the seeds' windows
-// -- does its rows on the plain path, status bits included.
+// -- does its rows on the plain path, status bits included.  Measured at 160,000 cells: 828 ->
+// 205 us, 1971 -> 119 FP64 instructions a warp (blocks of 16 rows; launch_gradients for 32).
 template <int NC>
 struct GradShared {
     static constexpr int CAP = 8 * NC;              // list entries: six a cell on average
@@ -1007,7 +1008,8 @@ __global__ void __launch_bounds__(BLOCK) k_time_step(phd_mesh M, const double *_
 // compared in FP32 first and only the cells within its rounding of the block's smallest
 // form theirs in FP64: 16 FP64 instructions fewer in the other warps, 100 left.  (Four threads a
 // cell, one a field, measured no faster at 16,000 cells and 99 us against 58 at 160,000: each
-// then forms dt A by itself.)  Measured at 160,000 cells: 90.6 -> 53.2 us.
+// then forms dt A by itself; with dt A handed round, 64.0 -> 63.4 us a step at 10,000 cells but 480 ->
+// 504 for two at 66,000.)  Measured at 160,000 cells: 90.6 -> 48.0 us.
 __global__ void __launch_bounds__(128) k_update_step(const __grid_constant__ phd_mesh M,
                                                      const __grid_constant__ phd_params P,
                                                      const double *__restrict__ flux, const double *__restrict__ cons,
