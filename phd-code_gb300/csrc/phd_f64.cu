@@ -787,7 +787,11 @@ __global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ phd_m
     const int n = M.n_cells, F = M.n_faces;
     if (m >= F) return;
     const int i = M.pair_i[m], j = M.pair_j[m];
-    if (i < 0 || i >= n || j < 0 || j >= n) { set_status(clk, PHD_STATUS_BAD_INDEX); return; }
+    if (i < 0 || i >= n || j < 0 || j >= n) {
+        pdl_wait();                                  // no kernel is done before the ones ahead of it
+        set_status(clk, PHD_STATUS_BAD_INDEX);
+        return;
+    }
     const bool boost = SOLVER == PHD_EXACT || P.boost != 0;
     const bool linear = P.reconstruction == PHD_LINEAR;
     Face64 A;
