@@ -352,8 +352,11 @@ class FluxStepper:
         if h is None:
             h = self._handover = L.PhdHandover32(twin=self.twin.data_ptr(), xmin=(ctypes.c_double * 2)(*dm.xmin[:2]),
                                                  xmax=(ctypes.c_double * 2)(*dm.xmax[:2]))
-            self._handover_out = L.geom32(self._geo_tensors(self.handover_records), out=True)
-        out = self._handover_out
+            self._handover_out = {}
+        records = bool(self.handover_records)         # may change from one hand-over to the next
+        out = self._handover_out.get(records)
+        if out is None:
+            out = self._handover_out[records] = L.geom32(self._geo_tensors(records), out=True)
         h.type, h.csr_work, h.bad = dm.type.data_ptr(), dm._csr_work.data_ptr(), dm._bad.data_ptr()
         h.periodic, h.dedup_periodic = int(dm.boundary == "periodic"), int(self.dedup_periodic)
         for k in ("face_ptr", "pair_j", "area32", "ct32", "x", "pair_dj", "list_len", "face32"):
@@ -371,8 +374,8 @@ class FluxStepper:
                 "phd_load_mesh_f32")
         if xr is None:
             self._x_real_valid = False
-        if self.records != self.handover_records:
-            self.records = self.handover_records
+        if self.records != records:
+            self.records = records
             self._set_geo()
         # what phd_load_mesh_f32 copied, counted from the arrays themselves
         nb = lambda k: pinned[k].numel() * pinned[k].element_size()

@@ -1,0 +1,38 @@
+"""``handover_records`` may change between compact hand-overs of equal counts: the records that a
+step reads are those of the mesh it runs on, so the steps equal, bit for bit, those of a stepper
+that never reads any."""
+import numpy as np
+import pytest
+import torch
+
+import phd_code_gb300 as pkg
+from _util import lattice_mesh, smooth_state
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("flags", [(False, True), (True, False, True), (False, True, False, True), (True, True, False)])
+@pytest.mark.parametrize("limiter", ["arepo", "tess"])
+def test_records_follow_the_attribute(flags, limiter):
+    mesh = lattice_mesh(14, "periodic", seed=3)
+    real = mesh.x[:, :mesh.n_real]
+    meshes = []
+    for k in range(len(flags)):               # generators moved too little to change a neighbour
+        moved = real + 1e-5 * (k + 1) * np.sin(7.0 * real[::-1])
+        m, order = pkg.meshgen.build_mesh(moved, "periodic", hilbert=False)
+        assert (m.n_cells, m.n_faces) == (mesh.n_cells, mesh.n_faces)
+        meshes.append(m)
+    kw = dict(gamma=1.4, solver="hllc", moving=True, precision="fp32", limiter=limiter)
+    a = pkg.FluxStepper(mesh, smooth_state(mesh), **kw)
+    b = pkg.FluxStepper(mesh, smooth_state(mesh), **kw)
+    for m, flag in zip(meshes, flags):
+        a.handover_records = flag
+        a.load_mesh(a.dmesh.pinned_host_compact(m))
+        b.load_mesh(b.dmesh.pinned_host_compact(m))
+        assert a.records == flag and (a.geo.entry_rec is not None) == flag
+        assert not b.records and b.geo.entry_rec is None
+        a.step(1)
+        b.step(1)
+        torch.cuda.synchronize()
+        assert torch.equal(a.cellrec, b.cellrec)
+        assert np.array_equal(a.cons_host(), b.cons_host())
