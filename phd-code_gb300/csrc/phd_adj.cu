@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(128, 3) k_adj_face(const __grid_constant__ phd
 }
 
 // Sum of row x's face contributions (12 values: primitives, gradients), in list order.
-__device__ __forceinline__ void gather_row(const phd_mesh &M, const double *__restrict__ face_adj, int x, double *s) {
+__device__ __forceinline__ void gather_row(const phd_mesh &M, const double *face_adj, int x, double *s) {
     const int F = M.n_faces;
 #pragma unroll
     for (int q = 0; q < 12; q++) s[q] = 0.0;
@@ -290,7 +290,7 @@ __device__ __forceinline__ void gather_row(const phd_mesh &M, const double *__re
 // 38 FP64 instructions an entry instead of 80.
 template <bool LINEAR>
 __global__ void __launch_bounds__(128) k_adj_cell(const __grid_constant__ phd_mesh M, phd_adj_index A, int limiter,
-                                                  const double *__restrict__ prim, const double *__restrict__ face_adj,
+                                                  const double *__restrict__ prim, const double *face_adj,
                                                   double *__restrict__ entry_adj /* [4][2F] */,
                                                   double *__restrict__ prim_part /* [4][n] */) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(128) k_adj_cell(const __grid_constant__ phd_me
 
 // Row x's sums of field f's face contributions (the primitive's, the gradient's two), in list
 // order, the loads of four faces at a time.
-__device__ __forceinline__ void gather_field(const phd_mesh &M, const double *__restrict__ face_adj, int x, int f,
+__device__ __forceinline__ void gather_field(const phd_mesh &M, const double *face_adj, int x, int f,
                                              double &s0, double &s1, double &s2) {
     const int F = M.n_faces, m0 = M.nbr_ptr[x], m1 = M.nbr_ptr[x + 1];
     s0 = s1 = s2 = 0.0;
@@ -500,7 +500,7 @@ __device__ __forceinline__ void gather_field(const phd_mesh &M, const double *__
 // with 415 FP64 instructions one behind the other (16,384 cells: 35.4 -> 23.5 us); the sums
 // keep their order.
 __global__ void __launch_bounds__(128) k_adj_cell_taped(const __grid_constant__ phd_mesh M, phd_adj_index A, int limiter,
-                                                        const double *__restrict__ face_adj,
+                                                        const double *face_adj,
                                                         double *__restrict__ entry_adj, double *__restrict__ prim_part,
                                                         const double *__restrict__ tape_f64,
                                                         const int32_t *__restrict__ tape_i32) {
@@ -599,8 +599,8 @@ __global__ void __launch_bounds__(128) k_adj_cell_taped(const __grid_constant__ 
 // rows of lam are zero.
 template <bool LINEAR>
 __global__ void __launch_bounds__(128) k_adj_final(const __grid_constant__ phd_mesh M, phd_adj_index A, double gamma,
-                                                   const double *__restrict__ cons, const double *__restrict__ prim_part,
-                                                   const double *__restrict__ entry_adj,
+                                                   const double *__restrict__ cons, const double *prim_part,
+                                                   const double *entry_adj,
                                                    const double *__restrict__ lam_next, double *__restrict__ lam) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= M.n_cells) return;

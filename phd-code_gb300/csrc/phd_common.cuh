@@ -30,8 +30,11 @@ struct NvtxRange {
 // with programmatic stream serialization) is scheduled once every block of this one has
 // called pdl_launch_dependents or left; pdl_wait blocks until every prerequisite grid has
 // completed and its memory operations are visible.  A kernel reads only data that no
-// earlier kernel of the step writes (the mesh) before pdl_wait.  Launched without the
-// attribute, both are no-ops in effect.
+// earlier kernel of the step writes (the mesh) before pdl_wait.  What one does write, it takes
+// through plain pointers: a const __restrict__ argument may be loaded through the read-only
+// path, which is for memory that stays as it is from the kernel's first block to its last,
+// and whose loads the clobber of pdl_wait need not hold back.  Launched without the attribute,
+// both are no-ops in effect.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -374,7 +374,7 @@ __device__ __forceinline__ void grad32_cell(int i, GradHead<REC> &H, const phd_m
                                             int moving, const EntrySrc &S,
                                             const int32_t *__restrict__ csr_nbr,
                                             const float4 *__restrict__ cell_geo,
-                                            const float4 *__restrict__ prim4, float4 *__restrict__ cellrec,
+                                            const float4 *prim4, float4 *__restrict__ cellrec,
                                             float2 *__restrict__ w2, phd_clock *clk) {
     const int c = H.c, e0 = H.e0, e1 = H.e1;
     if (c < 0) { set_status32(clk, PHD_STATUS_BAD_INDEX); return; }
@@ -499,7 +499,7 @@ template <int LIMITER, int ITEMS, bool REC>
 __global__ void __launch_bounds__(512) k_grad32(phd_mesh M, phd_params P, int moving, EntrySrc S,
                                                 const int32_t *__restrict__ csr_nbr,
                                                 const float4 *__restrict__ cell_geo,
-                                                const float4 *__restrict__ prim4, float4 *__restrict__ cellrec,
+                                                const float4 *prim4, float4 *__restrict__ cellrec,
                                                 float2 *__restrict__ w2, phd_clock *clk) {
     if (ITEMS == 0) {
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -701,16 +701,16 @@ __device__ __forceinline__ void gizmo_pair32(float sl, float sr, float qi4, floa
     xr = fminf(fmaxf(xr, fminf(orr, ir)), fmaxf(orr, ir));
 }
 
-// 64 bytes of a cell record in two 256-bit loads through the read-only path (the
-// record is not written while the face kernel runs).
-__device__ __forceinline__ void load_cellrec(const float4 *__restrict__ p, float4 &r0, float4 &r1, float4 &r2,
-                                             float4 &r3) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+// 64 bytes of a cell record in two 256-bit loads.  Not through the read-only path: the gradient
+// kernel still writes the records while the first blocks of this one are resident, ahead of
+// their wait, and volatile with a memory clobber keeps the loads behind it.
+__device__ __forceinline__ void load_cellrec(const float4 *p, float4 &r0, float4 &r1, float4 &r2, float4 &r3) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(r0.x), "=f"(r0.y), "=f"(r0.z), "=f"(r0.w), "=f"(r1.x), "=f"(r1.y), "=f"(r1.z), "=f"(r1.w)
-        : "l"(p));
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "l"(p) : "memory");
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(r2.x), "=f"(r2.y), "=f"(r2.z), "=f"(r2.w), "=f"(r3.x), "=f"(r3.y), "=f"(r3.z), "=f"(r3.w)
-        : "l"(p + 2));
+        : "l"(p + 2) : "memory");
 }
 
 // One face.  Linear reconstruction reads both cells' records (cellrec: primitives,
@@ -743,8 +743,8 @@ __device__ __forceinline__ FaceHead face_head(int m, const phd_mesh &M, const fl
 // the exact solver, which the reference runs boosted).
 template <int SOLVER, bool LINEAR, bool BOOST>
 __device__ __forceinline__ void face32_face(int m, const FaceHead &H, const phd_mesh &M, const phd_params &P,
-                                            int moving, const float4 *__restrict__ prim4,
-                                            const float4 *__restrict__ cellrec, const float2 *__restrict__ w2,
+                                            int moving, const float4 *prim4,
+                                            const float4 *cellrec, const float2 *w2,
                                             float4 *__restrict__ flux4, phd_clock *clocks,
                                             const int32_t *__restrict__ cell_run, const GasC &GC, float dt_run) {
     const int i = H.i, j = H.j;
@@ -837,8 +837,8 @@ template <int SOLVER, bool LINEAR, int ITEMS, bool BOOST>
 __global__ void __launch_bounds__(FACE_MAX_BLOCK, SOLVER == PHD_EXACT ? 1 : 5) k_face32(phd_mesh M, phd_params P, int moving,
                                                 const float4 *__restrict__ face_geo,
                                                 const float2 *__restrict__ face_ar,
-                                                const float4 *__restrict__ prim4,
-                                                const float4 *__restrict__ cellrec, const float2 *__restrict__ w2,
+                                                const float4 *prim4,
+                                                const float4 *cellrec, const float2 *w2,
                                                 float4 *__restrict__ flux4, phd_clock *clocks,
                                                 const int32_t *__restrict__ cell_run, const __grid_constant__ GasC GC) {
     if (ITEMS == 0) {
@@ -912,9 +912,9 @@ __device__ __forceinline__ UpdHead upd_head(int i, const phd_mesh &M, const int3
 template <bool PRE>
 __device__ __forceinline__ float update32_cell(int i, UpdHead &H, const phd_mesh &M, const phd_params &P,
                                                const int32_t *__restrict__ csr_face,
-                                               const float4 *__restrict__ flux4,
+                                               const float4 *flux4,
                                                const float4 *__restrict__ cell_geo,
-                                               const double *__restrict__ cons, double *__restrict__ cons_next,
+                                               const double *cons, double *__restrict__ cons_next,
                                                float4 *__restrict__ prim4, phd_clock *clocks,
                                                const int32_t *__restrict__ cell_run, float gam) {
     const int n = M.n_cells;
@@ -987,8 +987,8 @@ __device__ __forceinline__ float update32_cell(int i, UpdHead &H, const phd_mesh
 
 template <int ITEMS>
 __global__ void __launch_bounds__(512) k_update32(phd_mesh M, phd_params P, const int32_t *__restrict__ csr_face,
-                                                  const float4 *__restrict__ flux4, const float4 *__restrict__ cell_geo,
-                                                  const double *__restrict__ cons, double *__restrict__ cons_next,
+                                                  const float4 *flux4, const float4 *__restrict__ cell_geo,
+                                                  const double *cons, double *__restrict__ cons_next,
                                                   float4 *__restrict__ prim4, phd_clock *clocks,
                                                   const int32_t *__restrict__ cell_run, int n_runs) {
     const int n = M.n_cells;

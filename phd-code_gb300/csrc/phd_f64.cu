@@ -32,7 +32,7 @@ struct GradTape {
 // df (limited).  Returns status bits.  TAPE: also records the limiter's selections
 // (same arithmetic; only bookkeeping is added) when `record`.
 template <int DIM, bool TAPE = false>
-__device__ int cell_gradient_f64(const phd_mesh &M, const double *__restrict__ prim, int limiter,
+__device__ int cell_gradient_f64(const phd_mesh &M, const double *prim, int limiter,
                                  int c, double *df, GradTape tape = GradTape{nullptr, nullptr},
                                  bool record = false) {
     constexpr int NF = DIM + 2;
@@ -182,7 +182,7 @@ __device__ __noinline__ void generator_velocity_plain(const phd_mesh *M, const d
 
 // The same numbers with seeded quotients and roots; the sound speed only where a cell is off
 // its centroid far enough to be steered.
-__device__ __forceinline__ void generator_velocity(const phd_mesh &M, const double *__restrict__ prim, double gamma,
+__device__ __forceinline__ void generator_velocity(const phd_mesh &M, const double *prim, double gamma,
                                                    double eta, int regularize, int i, double *__restrict__ w) {
     const int n = M.n_cells;
     double wx[2] = {prim[(size_t)n + i], prim[2 * (size_t)n + i]};
@@ -341,7 +341,7 @@ __device__ __forceinline__ void gradient_changes(const GradShared<NC> &S, int k0
 }
 
 template <int NC, bool TAPE>
-__global__ void __launch_bounds__(4 * NC, 5) k_gradients(const __grid_constant__ phd_mesh M, const double *__restrict__ prim, int limiter,
+__global__ void __launch_bounds__(4 * NC, 5) k_gradients(const __grid_constant__ phd_mesh M, const double *prim, int limiter,
                                                       double *__restrict__ grad, phd_clock *clk, GradTape tape,
                                                       double *__restrict__ w, double gamma, double eta, int regularize) {
     __shared__ GradShared<NC> S;
@@ -579,8 +579,8 @@ __global__ void __launch_bounds__(4 * NC, 5) k_gradients(const __grid_constant__
 }
 
 template <int DIM>
-__device__ __forceinline__ void load_face_inputs(const phd_mesh &M, const double *__restrict__ prim,
-                                                 const double *__restrict__ grad, const double *__restrict__ face_w,
+__device__ __forceinline__ void load_face_inputs(const phd_mesh &M, const double *prim,
+                                                 const double *grad, const double *face_w,
                                                  int m, int i, int j, bool linear, double *pi, double *pj,
                                                  double *gi, double *gj, double *w) {
     constexpr int NF = DIM + 2;
@@ -632,8 +632,8 @@ __device__ __forceinline__ void load_geometry64(const phd_mesh &M, int m, int i,
         }
     }
 }
-__device__ __forceinline__ void load_values64(const phd_mesh &M, const double *__restrict__ prim,
-                                              const double *__restrict__ grad, int i, int j, bool linear, Face64 &A) {
+__device__ __forceinline__ void load_values64(const phd_mesh &M, const double *prim,
+                                              const double *grad, int i, int j, bool linear, Face64 &A) {
     const int n = M.n_cells;
 #pragma unroll
     for (int f = 0; f < 4; f++) { A.pi[f] = prim[(size_t)f * n + i]; A.pj[f] = prim[(size_t)f * n + j]; }
@@ -779,8 +779,8 @@ __device__ __noinline__ int face_flux_plain(const phd_mesh *M, const phd_params 
 template <int SOLVER>
 __global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ phd_mesh M, const __grid_constant__ phd_params P,
                                                    const __grid_constant__ Gas64 C, const __grid_constant__ Exact64 X,
-                                                   const double *__restrict__ prim,
-                                                   const double *__restrict__ grad, const double *__restrict__ w,
+                                                   const double *prim,
+                                                   const double *grad, const double *w,
                                                    double *__restrict__ face_w, double *__restrict__ flux,
                                                    phd_clock *clk) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1016,7 +1016,7 @@ __global__ void __launch_bounds__(BLOCK) k_time_step(phd_mesh M, const double *_
 // 504 for two at 66,000.)  Measured at 160,000 cells: 90.6 -> 48.0 us.
 __global__ void __launch_bounds__(128) k_update_step(const __grid_constant__ phd_mesh M,
                                                      const __grid_constant__ phd_params P,
-                                                     const double *__restrict__ flux, const double *__restrict__ cons,
+                                                     const double *flux, const double *cons,
                                                      double *__restrict__ cons_next, double *__restrict__ prim,
                                                      phd_clock *clk) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1119,7 +1119,7 @@ __global__ void __launch_bounds__(128) k_update_step(const __grid_constant__ phd
 // ---- mesh motion ------------------------------------------------------------------
 // Mesh.assign_generator_velocities mesh.pyx:397-426 (all cells), by itself: the plugin's stage,
 // and the steps without gradients.
-__global__ void __launch_bounds__(BLOCK) k_gen_vel(const __grid_constant__ phd_mesh M, const double *__restrict__ prim,
+__global__ void __launch_bounds__(BLOCK) k_gen_vel(const __grid_constant__ phd_mesh M, const double *prim,
                                                    double gamma, double eta, int regularize, double *__restrict__ w) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
