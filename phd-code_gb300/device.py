@@ -382,17 +382,22 @@ class DeviceMesh:
 
 
 class DeviceClock:
-    """Device ``phd_clock``: dt, t, t_end, CFL accumulator and status bits."""
+    """Device ``phd_clock``: dt, t, t_end, CFL accumulator and status bits.
 
-    def __init__(self, device="cuda", dt=0.0, t=0.0, t_end=0.0):
+    A new clock is complete when its constructor returns, whatever stream reads it first.
+    ``in_stream`` leaves a clock at rest to two fills in the order of the current stream
+    instead: for callers that go on there."""
+
+    def __init__(self, device="cuda", dt=0.0, t=0.0, t_end=0.0, in_stream=False):
         self.device = _dev(device)
-        words = torch.zeros(L.CLOCK_BYTES // 8, dtype=torch.int64, device=self.device)
-        self.buf = words.view(torch.uint8)
-        if dt == 0.0 and t == 0.0 and t_end == 0.0:
-            # at rest: all zero but the CFL accumulator (infinity), filled in on the device, where
-            # a host copy would wait for the copy engine
+        if in_stream and dt == 0.0 and t == 0.0 and t_end == 0.0:
+            # all zero but the CFL accumulator (infinity); a host copy would wait for the stream
+            # and the copy engine
+            words = torch.zeros(L.CLOCK_BYTES // 8, dtype=torch.int64, device=self.device)
             words[L.PhdClock.dtmin_bits.offset // 8].fill_(0x7ff0000000000000)
+            self.buf = words.view(torch.uint8)
         else:
+            self.buf = torch.empty(L.CLOCK_BYTES, dtype=torch.uint8, device=self.device)
             self.set(dt=dt, t=t, t_end=t_end)
 
     def set(self, dt=0.0, t=0.0, t_end=0.0, status=0, step=0):

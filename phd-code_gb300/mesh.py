@@ -108,7 +108,7 @@ class Mesh:
         mass or energy (reads the device status, one small device-to-host copy)."""
         from .device import DeviceClock
         dm = self._need()
-        clk = clock or DeviceClock(particles.device)
+        clk = clock or DeviceClock(particles.device, in_stream=True)
         L.check(L.lib().phd_update_from_fluxes_f64(dm.ref, L.ptr(riemann.fluxes.block("flux")), float(dt),
                                                    L.ptr(particles.block("conservative")), clk.ptr,
                                                    L.stream_handle()), "phd_update_from_fluxes_f64")

@@ -127,7 +127,7 @@ class PieceWiseLinear(ReconstructionBase):
         if self.grad is None:
             self.initialize(particles.device)
         self.grad.resize(dm.n_cells)
-        clk = clock or DeviceClock(particles.device)
+        clk = clock or DeviceClock(particles.device, in_stream=True)
         L.check(L.lib().phd_gradients_f64(dm.ref, L.ptr(particles.block("primitive")), self.slope_limiter,
                                           L.ptr(self.grad.block("primitive")), clk.ptr, L.stream_handle()),
                 "phd_gradients_f64")

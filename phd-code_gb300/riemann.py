@@ -44,7 +44,7 @@ class RiemannBase:
         if self.fluxes is None:
             self.initialize(particles.device)
         self.fluxes.resize(dm.n_faces)
-        clk = clock or DeviceClock(particles.device)
+        clk = clock or DeviceClock(particles.device, in_stream=True)
         L.check(L.lib().phd_riemann_f64(dm.ref, self.solver, eos.get_gamma(), int(bool(self.boost)), 1000,
                                         L.ptr(reconstruction.left_states.block("primitive")),
                                         L.ptr(reconstruction.right_states.block("primitive")),
@@ -59,7 +59,7 @@ class RiemannBase:
         if mesh is None:
             mesh = getattr(particles, "_mesh", None)
         dm = mesh._need()
-        clk = clock or DeviceClock(particles.device)
+        clk = clock or DeviceClock(particles.device, in_stream=True)
         L.check(L.lib().phd_time_step_f64(dm.ref, L.ptr(particles.block("primitive")), eos.get_gamma(),
                                           self.cfl, int(bool(self.boost)), 0, clk.ptr, L.stream_handle()),
                 "phd_time_step_f64")

@@ -35,16 +35,25 @@ class FluxStepper:
         self.device = torch.device(device)
         self.handover_records = bool(handover_records)
         self.records = False        # entry_rec holds the current mesh's records
+        self.stream = stream
+        if stream is not None:
+            # all below is allocated, filled and launched on the stepper's stream, after what the
+            # caller has in flight: nothing else orders the fills and that stream's kernels
+            stream.wait_stream(torch.cuda.current_stream(self.device))
+        with torch.cuda.stream(stream):
+            self._set_up(mesh, prim, make_params(gamma=gamma, cfl=cfl, eta=eta, reconstruction=reconstruction,
+                                                 limiter=limiter, gizmo=gizmo, solver=solver, boost=boost,
+                                                 regularize=regularize),
+                         moving, precision, t_end, face_velocity, dedup_periodic)
+
+    def _set_up(self, mesh, prim, params, moving, precision, t_end, face_velocity, dedup_periodic):
         self.dmesh = mesh if isinstance(mesh, DeviceMesh) else DeviceMesh(mesh, device=self.device)
         dm = self.dmesh
-        self.params = make_params(gamma=gamma, cfl=cfl, eta=eta, reconstruction=reconstruction,
-                                  limiter=limiter, gizmo=gizmo, solver=solver, boost=boost,
-                                  regularize=regularize)
+        self.params = params
         self.moving = bool(moving)
         if precision not in ("fp64", "fp32"):
             raise ValueError("precision must be 'fp64' or 'fp32'")
         self.precision = precision
-        self.stream = stream
         self.dedup_periodic = bool(dedup_periodic)
         self.launch = None          # FP32 launch shapes (PhdLaunch, e.g. from autotune.tune)
         n, F, d = dm.n_cells, dm.n_faces, dm.dim
@@ -56,10 +65,10 @@ class FluxStepper:
             raise ValueError("prim must be [%d][%d]" % (nf, n))
         self.cons = torch.empty((nf, n), dtype=f64, device=dev)
         self.cons_next = torch.empty((nf, n), dtype=f64, device=dev)
-        self.clock = DeviceClock(dev, t_end=t_end)
+        self.clock = DeviceClock(dev, t_end=t_end, in_stream=True)
         self._graph = None
         self._graph_steps = 0
-        s = L.stream_handle(stream)
+        s = L.stream_handle(self.stream)
         lib = L.lib()
         L.check(lib.phd_cons_from_prim_f64(d, n, self.params.gamma, L.ptr(dm.vol), L.ptr(self.prim),
                                            L.ptr(self.cons), s), "phd_cons_from_prim_f64")
