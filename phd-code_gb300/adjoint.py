@@ -14,6 +14,7 @@ one segment).
 ``prim0``.
 """
 import ctypes
+import weakref
 
 import numpy as np
 import torch
@@ -90,6 +91,17 @@ class _MeshBuffers:
         return self.work
 
 
+class _Tail:
+    """The last segment's states from a forward pass that kept them, for one backward pass."""
+
+    def __init__(self, states):
+        self.states = states
+
+    def take(self):
+        states, self.states = self.states, None
+        return states
+
+
 class FluxRunRecord:
     """A recorded run: the per-step records and the options of the step.
 
@@ -122,7 +134,14 @@ class FluxRunRecord:
         self._clocks0 = torch.as_tensor(np.stack(rows)).to(self.device)
         self.clocks = self._clocks0.clone()
         self._bufs = {}
-        self._tail = None                    # the last segment's states, from a forward that kept them
+        self._kept = None                    # the _Tail of a forward pass asked to keep one
+        self._kept_ref = None                # and that of the newest pass, whoever holds it
+
+    @property
+    def _tail(self):
+        """The newest forward pass's last segment while it is held and not yet used."""
+        kept = self._kept_ref() if self._kept_ref is not None else None
+        return None if kept is None else kept.states
 
     def _buffers(self, dm):
         b = self._bufs.get(id(dm))
@@ -226,10 +245,10 @@ class FluxRunRecord:
         a sixth of a pass over two segments (12.4 -> 10.8 ms, 40 steps at 128 x 128)."""
         self.clocks.copy_(self._clocks0)
         self.ckpt = {0: U0.clone()}
-        self._tail = None
+        self._kept = self._kept_ref = None
         N = len(self.steps)
         tail = self._tail_start() if keep else N
-        prev = None
+        prev = kept = None
         for k, rec in enumerate(self.steps):
             dm = rec.dmesh
             b = self._buffers(dm)
@@ -238,7 +257,8 @@ class FluxRunRecord:
             elif prev is not b:
                 self._load_real(dm, prev.cons[:, :dm.n_real], b.cons, b.prim)
             if k == tail:
-                self._tail, cons = self._segment(k, N, b.cons.clone(), b.prim.clone(), True)
+                states, cons = self._segment(k, N, b.cons.clone(), b.prim.clone(), True)
+                kept = _Tail(states)
                 break
             self._step(k, b.prim, b.cons, b.nxt, b.grad)
             b.cons, b.nxt = b.nxt, b.cons
@@ -251,6 +271,8 @@ class FluxRunRecord:
         for row in self.clocks.cpu().numpy():
             st |= L.PhdClock.from_buffer_copy(row.tobytes()).status
         L.raise_status(st)
+        if kept is not None:
+            self._kept, self._kept_ref = kept, weakref.ref(kept)
         return UT
 
     # --- branch-frozen forward (finite differences on the branch the run takes) ----
@@ -306,10 +328,10 @@ class FluxRunRecord:
         self._load_real(dm, U_real, c, p)
         return c, p
 
-    def _replay_segment(self, a, b):
+    def _replay_segment(self, a, b, ckpt=None):
         """Recompute the all-cell states entering steps a..b-1 from the checkpoint at a."""
         self.clocks[a:b].copy_(self._clocks0[a:b])      # each step's CFL finish overwrote its dt
-        return self._segment(a, b, *self._loaded(self.steps[a].dmesh, self.ckpt[a]))[0]
+        return self._segment(a, b, *self._loaded(self.steps[a].dmesh, (self.ckpt if ckpt is None else ckpt)[a]))[0]
 
     def _segment(self, a, b, cons, prim, finish=False):
         """The all-cell states (totals, primitives, gradients and the gradients' limiter tape)
@@ -340,18 +362,21 @@ class FluxRunRecord:
                                                     L.stream_handle()), "gradients")
         return states, cons
 
-    def backward(self, lam_T):
-        """dLoss/dU_0 from dLoss/dU_T, segment by segment (recompute from checkpoints)."""
+    def backward(self, lam_T, ckpt=None, kept=None):
+        """dLoss/dU_0 from dLoss/dU_T, segment by segment (recompute from checkpoints): of the
+        newest forward pass, or of the one whose checkpoints and kept segment are given."""
         lam = lam_T
+        if ckpt is None:
+            ckpt, kept = self.ckpt, self._kept
         N = len(self.steps)
         prev = None                                     # the buffers whose lam is current
-        starts = sorted(self.ckpt)
+        starts = sorted(ckpt)
         for si in range(len(starts) - 1, -1, -1):
             a = starts[si]
             b = starts[si + 1] if si + 1 < len(starts) else N
-            states, self._tail = self._tail if b == N else None, None
+            states = kept.take() if b == N and kept is not None else None
             if states is None:
-                states = self._replay_segment(a, b)
+                states = self._replay_segment(a, b, ckpt)
             for k in range(b - 1, a - 1, -1):
                 rec = self.steps[k]
                 bufs = self._buffers(rec.dmesh)
@@ -372,7 +397,10 @@ def cons_from_prim_t(prim, vol, gamma):
 
 
 class FluxRun(torch.autograd.Function):
-    """prim0 [4][n_real] -> final densities [n_real] through a recorded run."""
+    """prim0 [4][n_real] -> final densities [n_real] through a recorded run.
+
+    A pass's checkpoints and kept segment go with its graph, so that each backward pass is of
+    its own forward pass, and what a graph held is given back with it."""
 
     @staticmethod
     def forward(ctx, prim0, run):
@@ -380,7 +408,8 @@ class FluxRun(torch.autograd.Function):
         with torch.no_grad():
             U0 = cons_from_prim_t(prim0, vol0, run.params.gamma)
             UT = run.forward(U0.contiguous(), keep=ctx.needs_input_grad[0])
-        ctx.run = run
+        ctx.run, ctx.ckpt, ctx.kept = run, run.ckpt, run._kept
+        run._kept = None                                # the graph's alone
         ctx.save_for_backward(prim0)
         return UT[0] / run.final_vol
 
@@ -390,7 +419,7 @@ class FluxRun(torch.autograd.Function):
         (prim0,) = ctx.saved_tensors
         lam_T = torch.zeros((4, run.n_real), dtype=F64, device=prim0.device)
         lam_T[0] = g_rho / run.final_vol
-        lam0 = run.backward(lam_T)
+        lam0 = run.backward(lam_T, ctx.ckpt, ctx.kept)
         vol0 = run.steps[0].dmesh.vol[:run.n_real]
         # cons_from_prim is local and smooth: its vector-Jacobian product via autograd
         with torch.enable_grad():
