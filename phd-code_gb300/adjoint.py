@@ -402,12 +402,18 @@ class FluxRun(torch.autograd.Function):
     A pass's checkpoints and kept segment go with its graph, so that each backward pass is of
     its own forward pass, and what a graph held is given back with it."""
 
+    @classmethod
+    def apply(cls, prim0, run):
+        # in forward the grad mode is off and needs_input_grad is the leaf's own, with or
+        # without no_grad: asked here
+        return super().apply(prim0, run, torch.is_grad_enabled())
+
     @staticmethod
-    def forward(ctx, prim0, run):
+    def forward(ctx, prim0, run, grad_mode):
         vol0 = run.steps[0].dmesh.vol[:run.n_real]
         with torch.no_grad():
             U0 = cons_from_prim_t(prim0, vol0, run.params.gamma)
-            UT = run.forward(U0.contiguous(), keep=ctx.needs_input_grad[0])
+            UT = run.forward(U0.contiguous(), keep=grad_mode and ctx.needs_input_grad[0])
         ctx.run, ctx.ckpt, ctx.kept = run, run.ckpt, run._kept
         run._kept = None                                # the graph's alone
         ctx.save_for_backward(prim0)
@@ -426,4 +432,4 @@ class FluxRun(torch.autograd.Function):
             p = prim0.detach().requires_grad_(True)
             U = cons_from_prim_t(p, vol0, run.params.gamma)
             (gp,) = torch.autograd.grad(U, p, grad_outputs=lam0)
-        return gp, None
+        return gp, None, None

@@ -54,3 +54,18 @@ def test_a_dropped_graph_takes_its_record_with_it():
     del out
     gc.collect()
     assert run._tail is None
+
+
+def test_no_record_without_a_gradient(monkeypatch):
+    run, p0 = _run(5, 20)
+    taped = []
+    step = FluxRunRecord._step
+    monkeypatch.setattr(FluxRunRecord, "_step",
+                        lambda self, k, *a, **kw: (taped.append(len(a) > 4 and a[4] is not None), step(self, k, *a, **kw))[1])
+    p = p0.clone().requires_grad_(True)
+    with torch.no_grad():
+        rho = FluxRun.apply(p, run)
+    assert run._tail is None and not any(taped)
+    assert torch.equal(rho, FluxRun.apply(p0, run)) and not any(taped)
+    out = FluxRun.apply(p, run)
+    assert torch.equal(out.detach(), rho) and any(taped) and run._tail is not None
