@@ -1176,12 +1176,13 @@ inline void launch_face_flux(const phd_mesh &M, const phd_params &P, const doubl
     const int block = M.n_faces < 16 * 128 * sm_count_current() ? 32 : 128, grid = grid_for_block(M.n_faces, block);
     const Gas64 C = gas64(P.gamma);
     const Exact64 X = exact64(P.gamma);
-    if (P.solver == PHD_HLL)
-        launch_pdl(k_face_flux<PHD_HLL>, grid, block, queue, M, P, C, X, prim, grad, w, face_w, flux, clk);
+    // a number without a name is HLL, as riemann_flux has it
+    if (P.solver == PHD_EXACT)
+        launch_pdl(k_face_flux<PHD_EXACT>, grid, block, queue, M, P, C, X, prim, grad, w, face_w, flux, clk);
     else if (P.solver == PHD_HLLC)
         launch_pdl(k_face_flux<PHD_HLLC>, grid, block, queue, M, P, C, X, prim, grad, w, face_w, flux, clk);
     else
-        launch_pdl(k_face_flux<PHD_EXACT>, grid, block, queue, M, P, C, X, prim, grad, w, face_w, flux, clk);
+        launch_pdl(k_face_flux<PHD_HLL>, grid, block, queue, M, P, C, X, prim, grad, w, face_w, flux, clk);
 }
 
 inline int launch_status() {
