@@ -1093,10 +1093,13 @@ __global__ void __launch_bounds__(128) k_update_step(const __grid_constant__ phd
             prim[(size_t)q * n + i] = p[q];
         }
         if (real) {
-            // R/c within a few FP32 roundings while the operands are well inside FP32's range
+            // R/c within a few FP32 roundings while the operands and p/rho are well inside FP32's
+            // range (where the quotient is subnormal its rounding could hide the smallest)
             const unsigned lo = (1023u - 100u) << 20, span = 200u << 20;
-            const bool in = f64_hi(p[0]) - lo < span && f64_hi(p[3]) - lo < span && f64_hi(vol) - lo < span;
-            const float cs = sqrtf((float)P.gamma * f64_to_f32(p[3]) / f64_to_f32(p[0]));
+            const float c2 = (float)P.gamma * f64_to_f32(p[3]) / f64_to_f32(p[0]);
+            const bool in = f64_hi(p[0]) - lo < span && f64_hi(p[3]) - lo < span && f64_hi(vol) - lo < span &&
+                            c2 >= 7.8886091e-31f;
+            const float cs = sqrtf(c2);
             const float vx = f64_to_f32(p[1]), vy = f64_to_f32(p[2]);
             const float den = boost ? cs : cs + sqrtf(vx * vx + vy * vy);
             c32 = in ? sqrtf(f64_to_f32(vol) * 0.3183098861837907f) / den : -1.f;
