@@ -253,8 +253,9 @@ class FluxStepper:
             self._side = torch.cuda.Stream(self.device)
             self._side2 = torch.cuda.Stream(self.device)
             self._ev = [torch.cuda.Event() for _ in range(8)]
+            main = self._main_stream()
             for e in self._ev:                        # creates the events' handles
-                e.record(self._main_stream())
+                e.record(main)
             self._ev_handles = (ctypes.c_void_p * 8)(*(e.cuda_event for e in self._ev))
             self._side_handles = (ctypes.c_void_p * 2)(self._side.cuda_stream, self._side2.cuda_stream)
         if compact:
