@@ -113,16 +113,16 @@ class FluxStepper:
         """The step's geometry: with entry_rec only while it holds the current mesh's."""
         self.geo = L.geom32(self._geo_tensors(self.records))
 
-    def build_entry_records(self):
+    def build_entry_records(self, stream=None):
         """(FP32) Write the per-entry gradient records of the current mesh, so the steps
         that follow read them instead of forming them from the faces (the same bits,
         about 8 us less per step at 1M cells; the build costs about as much as 7 steps
-        save).  A no-op when they are current."""
+        save).  A no-op when they are current.  On the stepper's stream, or the given one."""
         if self.precision != "fp32" or self.records:
             return
         out = L.geom32(self._geo_tensors(), out=True)
         L.check(L.lib().phd_prepare_f32_parts(self.dmesh.ref, None, ctypes.byref(out), L.PREP_RECORDS,
-                                              L.stream_handle(self.stream)), "phd_prepare_f32_parts")
+                                              L.stream_handle(stream or self.stream)), "phd_prepare_f32_parts")
         self.records = True
         self._set_geo()
 
@@ -509,6 +509,11 @@ class FluxStepper:
         return g
 
     def replay(self):
+        """Launch the captured steps on the current stream.  They read the gradient records, which
+        a hand-over since may have left unwritten: those of the mesh as it is now are built
+        first."""
+        if self.precision == "fp32" and not self.records:
+            self.build_entry_records(torch.cuda.current_stream(self.device))
         self._graph.replay()
 
     # ------------------------------------------------------------------------------

@@ -36,3 +36,23 @@ def test_records_follow_the_attribute(flags, limiter):
         torch.cuda.synchronize()
         assert torch.equal(a.cellrec, b.cellrec)
         assert np.array_equal(a.cons_host(), b.cons_host())
+
+
+@pytest.mark.parametrize("compact", [True, False])
+def test_a_captured_graph_reads_the_new_meshs_records(compact):
+    """A graph outlives a hand-over of equal counts; its steps read records, and a replay builds those
+    that the hand-over left unwritten."""
+    mesh = lattice_mesh(14, "periodic", seed=3)
+    real = mesh.x[:, :mesh.n_real]
+    other, _ = pkg.meshgen.build_mesh(real + 1e-5 * np.sin(7.0 * real[::-1]), "periodic", hilbert=False)
+    assert (other.n_cells, other.n_faces) == (mesh.n_cells, mesh.n_faces)
+    a, b = (pkg.FluxStepper(mesh, smooth_state(mesh), gamma=1.4, moving=True, precision="fp32") for _ in range(2))
+    a.capture(2)
+    for st in (a, b):
+        st.load_mesh(st.dmesh.pinned_host_compact(other) if compact else st.dmesh.pinned_host(other))
+    assert not a.records
+    for _ in range(2):
+        a.replay()
+        b.step(2)
+        torch.cuda.synchronize()
+        assert a.records and np.array_equal(a.cons_host(), b.cons_host())
