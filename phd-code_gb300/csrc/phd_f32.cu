@@ -1157,7 +1157,7 @@ int cells_prim_f32(const phd_mesh *mesh, const phd_params *par, const phd_geom32
 }
 
 template <int SOLVER, int ITEMS>
-void launch_face32_items(bool linear, int grid, int block, PdlQueue &s, const phd_mesh &M, const phd_params &P,
+void launch_face32_items(bool linear, int grid, int block, PdlQueue &queue, const phd_mesh &M, const phd_params &P,
                          int moving, const phd_geom32 *G, const float4 *prim4, const float4 *cellrec, const float2 *w2,
                          float4 *flux4, phd_clock *clocks, const int32_t *cell_run) {
     const float4 *fg = reinterpret_cast<const float4 *>(G->face_geo);
@@ -1166,17 +1166,17 @@ void launch_face32_items(bool linear, int grid, int block, PdlQueue &s, const ph
     constexpr bool EX = SOLVER == PHD_EXACT;      // the exact solver always works boosted
     if (EX || P.boost) {
         if (linear)
-            launch_pdl(k_face32<SOLVER, true, ITEMS, true>, grid, block, s, M, P, moving, fg, fa, prim4, cellrec, w2,
+            launch_pdl(k_face32<SOLVER, true, ITEMS, true>, grid, block, queue, M, P, moving, fg, fa, prim4, cellrec, w2,
                        flux4, clocks, cell_run, gc);
         else
-            launch_pdl(k_face32<SOLVER, false, ITEMS, true>, grid, block, s, M, P, moving, fg, fa, prim4, cellrec, w2,
+            launch_pdl(k_face32<SOLVER, false, ITEMS, true>, grid, block, queue, M, P, moving, fg, fa, prim4, cellrec, w2,
                        flux4, clocks, cell_run, gc);
     } else if constexpr (!EX) {
         if (linear)
-            launch_pdl(k_face32<SOLVER, true, ITEMS, false>, grid, block, s, M, P, moving, fg, fa, prim4, cellrec,
+            launch_pdl(k_face32<SOLVER, true, ITEMS, false>, grid, block, queue, M, P, moving, fg, fa, prim4, cellrec,
                        w2, flux4, clocks, cell_run, gc);
         else
-            launch_pdl(k_face32<SOLVER, false, ITEMS, false>, grid, block, s, M, P, moving, fg, fa, prim4, cellrec,
+            launch_pdl(k_face32<SOLVER, false, ITEMS, false>, grid, block, queue, M, P, moving, fg, fa, prim4, cellrec,
                        w2, flux4, clocks, cell_run, gc);
     }
 }
@@ -1184,20 +1184,20 @@ void launch_face32_items(bool linear, int grid, int block, PdlQueue &s, const ph
 // The exact solver's face kernel is bound by the FP64 pipe and holds 120+ registers:
 // it runs one face per thread whatever the requested items.
 template <int SOLVER>
-void launch_face32(bool linear, int items, int grid, int block, PdlQueue &s, const phd_mesh &M,
+void launch_face32(bool linear, int items, int grid, int block, PdlQueue &queue, const phd_mesh &M,
                    const phd_params &P, int moving, const phd_geom32 *G, const float4 *prim4, const float4 *cellrec,
                    const float2 *w2, float4 *flux4, phd_clock *clocks, const int32_t *cell_run) {
     if (items == 0)
-        launch_face32_items<SOLVER, 0>(linear, grid, block, s, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
+        launch_face32_items<SOLVER, 0>(linear, grid, block, queue, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
                                        cell_run);
     else if (SOLVER == PHD_EXACT || items == 1)
-        launch_face32_items<SOLVER, 1>(linear, grid, block, s, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
+        launch_face32_items<SOLVER, 1>(linear, grid, block, queue, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
                                        cell_run);
     else if (items == 2)
-        launch_face32_items<SOLVER, 2>(linear, grid, block, s, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
+        launch_face32_items<SOLVER, 2>(linear, grid, block, queue, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
                                        cell_run);
     else
-        launch_face32_items<SOLVER, 4>(linear, grid, block, s, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
+        launch_face32_items<SOLVER, 4>(linear, grid, block, queue, M, P, moving, G, prim4, cellrec, w2, flux4, clocks,
                                        cell_run);
 }
 
@@ -1243,33 +1243,33 @@ inline bool items_ok(int k) { return k == 0 || k == 1 || k == 2 || k == 4; }
 inline int items_of(int k) { return k <= 1 ? 1 : k; }
 
 template <int LIMITER>
-void launch_grad32_rec(int items, int grid, int block, PdlQueue &s, const phd_mesh &M, const phd_params &P,
+void launch_grad32_rec(int items, int grid, int block, PdlQueue &queue, const phd_mesh &M, const phd_params &P,
                        int moving, const EntrySrc &S, const int32_t *csr_nbr, const float4 *cg, const float4 *p4,
                        float4 *cr, float2 *w, phd_clock *clocks) {
     if (items == 0)
-        launch_pdl(k_grad32<LIMITER, 0, true>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+        launch_pdl(k_grad32<LIMITER, 0, true>, grid, block, queue, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else if (items == 1)
-        launch_pdl(k_grad32<LIMITER, 1, true>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+        launch_pdl(k_grad32<LIMITER, 1, true>, grid, block, queue, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else if (items == 2)
-        launch_pdl(k_grad32<LIMITER, 2, true>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+        launch_pdl(k_grad32<LIMITER, 2, true>, grid, block, queue, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else
-        launch_pdl(k_grad32<LIMITER, 4, true>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+        launch_pdl(k_grad32<LIMITER, 4, true>, grid, block, queue, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
 }
 
-// without entry records (S.entry_rec null): one item per thread, the records formed
+// without entry records (S.entry_rec null): at most two items per thread, the records formed
 // from the faces (the launch a freshly handed-over mesh's first step takes)
 template <int LIMITER>
-void launch_grad32(int items, int grid, int block, PdlQueue &s, const phd_mesh &M, const phd_params &P, int moving,
+void launch_grad32(int items, int grid, int block, PdlQueue &queue, const phd_mesh &M, const phd_params &P, int moving,
                    const EntrySrc &S, const int32_t *csr_nbr, const float4 *cg, const float4 *p4, float4 *cr,
                    float2 *w, phd_clock *clocks) {
     if (S.entry_rec)
-        launch_grad32_rec<LIMITER>(items, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+        launch_grad32_rec<LIMITER>(items, grid, block, queue, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else if (items == 0)
-        launch_pdl(k_grad32<LIMITER, 0, false>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+        launch_pdl(k_grad32<LIMITER, 0, false>, grid, block, queue, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else if (items == 1)
-        launch_pdl(k_grad32<LIMITER, 1, false>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+        launch_pdl(k_grad32<LIMITER, 1, false>, grid, block, queue, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
     else
-        launch_pdl(k_grad32<LIMITER, 2, false>, grid, block, s, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
+        launch_pdl(k_grad32<LIMITER, 2, false>, grid, block, queue, M, P, moving, S, csr_nbr, cg, p4, cr, w, clocks);
 }
 
 inline int g32(int n) { return n > 0 ? (n + B32 - 1) / B32 : 1; }
@@ -1292,7 +1292,7 @@ using namespace phd;
 static int step_f32(const phd_mesh *mesh, const phd_geom32 *geo, const phd_params *par, int32_t moving,
                          const phd_launch *launch, float *prim4, const double *cons, double *cons_next, float *cellrec,
                          float *w2, float *flux4, phd_clock *clocks, int32_t n_runs, const int32_t *cell_run,
-                         PdlQueue &stream, cudaEvent_t *marks) {
+                         PdlQueue &queue, cudaEvent_t *marks) {
     if (!mesh || mesh->dim != 2 || !geo || !par || !prim4 || !cons || !cons_next || !flux4 || !clocks)
         return PHD_ERR_ARG;
     const bool linear = par->reconstruction == PHD_LINEAR;
@@ -1332,46 +1332,46 @@ static int step_f32(const phd_mesh *mesh, const phd_geom32 *geo, const phd_param
                          M.n_faces};
     const float4 *cg = reinterpret_cast<const float4 *>(geo->cell_geo);
     const int32_t *runs = n_runs > 1 ? cell_run : nullptr;
-    if (marks) cudaEventRecord(marks[0], stream.stream);
+    if (marks) cudaEventRecord(marks[0], queue.stream);
     if (linear || moving) {
         if (par->limiter == PHD_LIMITER_TESS)
-            launch_grad32<PHD_LIMITER_TESS>(kg, gc, L.block_grad, stream, M, *par, (int)moving, er, geo->csr_nbr, cg,
+            launch_grad32<PHD_LIMITER_TESS>(kg, gc, L.block_grad, queue, M, *par, (int)moving, er, geo->csr_nbr, cg,
                                             p4, cr, w, clocks);
         else
-            launch_grad32<PHD_LIMITER_AREPO>(kg, gc, L.block_grad, stream, M, *par, (int)moving, er, geo->csr_nbr, cg,
+            launch_grad32<PHD_LIMITER_AREPO>(kg, gc, L.block_grad, queue, M, *par, (int)moving, er, geo->csr_nbr, cg,
                                              p4, cr, w, clocks);
     }
-    if (marks) cudaEventRecord(marks[1], stream.stream);
+    if (marks) cudaEventRecord(marks[1], queue.stream);
     if (M.n_faces) {
         switch (par->solver) {
             case PHD_HLL:
-                launch_face32<PHD_HLL>(linear, kf, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx, clocks,
+                launch_face32<PHD_HLL>(linear, kf, gf, L.block_face, queue, M, *par, moving, geo, p4, cr, w, fx, clocks,
                                        runs);
                 break;
             case PHD_HLLC:
-                launch_face32<PHD_HLLC>(linear, kf, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx, clocks,
+                launch_face32<PHD_HLLC>(linear, kf, gf, L.block_face, queue, M, *par, moving, geo, p4, cr, w, fx, clocks,
                                         runs);
                 break;
             default:
-                launch_face32<PHD_EXACT>(linear, kf, gf, L.block_face, stream, M, *par, moving, geo, p4, cr, w, fx,
+                launch_face32<PHD_EXACT>(linear, kf, gf, L.block_face, queue, M, *par, moving, geo, p4, cr, w, fx,
                                          clocks, runs);
                 break;
         }
     }
-    if (marks) cudaEventRecord(marks[2], stream.stream);
+    if (marks) cudaEventRecord(marks[2], queue.stream);
     if (ku == 0)
-        launch_pdl(k_update32<0>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
+        launch_pdl(k_update32<0>, gu, L.block_update, queue, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
                    cons_next, p4, clocks, runs, (int)n_runs);
     else if (ku == 1)
-        launch_pdl(k_update32<1>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
+        launch_pdl(k_update32<1>, gu, L.block_update, queue, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
                    cons_next, p4, clocks, runs, (int)n_runs);
     else if (ku == 2)
-        launch_pdl(k_update32<2>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
+        launch_pdl(k_update32<2>, gu, L.block_update, queue, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
                    cons_next, p4, clocks, runs, (int)n_runs);
     else
-        launch_pdl(k_update32<4>, gu, L.block_update, stream, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
+        launch_pdl(k_update32<4>, gu, L.block_update, queue, M, *par, geo->csr_face, (const float4 *)fx, cg, cons,
                    cons_next, p4, clocks, runs, (int)n_runs);
-    if (marks) cudaEventRecord(marks[3], stream.stream);
+    if (marks) cudaEventRecord(marks[3], queue.stream);
     return cudaPeekAtLastError() == cudaSuccess ? PHD_OK : PHD_ERR_LAUNCH;
 }
 

@@ -263,7 +263,7 @@ __device__ __noinline__ int gradient_row_plain(const phd_mesh *M, const double *
 // A block that meets anything unusual -- an index out of range, a cell that its face does not
 // name, more list entries than the shared arrays hold, an operand outside the seeds' windows
 // -- does its rows on the plain path, status bits included.  Measured at 160,000 cells: 828 ->
-// 205 us, 1971 -> 119 FP64 instructions a warp (blocks of 16 rows; launch_gradients for 32).
+// 162 us, 1971 -> 104 FP64 instructions a warp (of 32 rows before, of 8 now), 70% of the pipe.
 template <int NC>
 struct GradShared {
     static constexpr int CAP = 8 * NC;              // list entries: six a cell on average

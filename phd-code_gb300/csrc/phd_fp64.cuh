@@ -3,10 +3,12 @@
 // GB300 issues one FP64 warp instruction per 19 clocks and SM, whatever the number of
 // active lanes, against 0.3 clocks for an FP32 or integer one (measured: fused
 // multiply-add, addition, product and comparison alike); a division or square root of the
-// compiler takes 141-143 clocks, 7.5 FP64 instructions.  The FP64 kernels keep that pipe
-// 80-85% busy, so their time is their count of FP64 instructions, and 40-odd FP32 and integer
-// instructions run in the shadow of each.  The helpers here therefore form everything that
-// need not be an FP64 instruction with FP32 and integer ones:
+// compiler takes 141-143 clocks, 7.5 FP64 instructions.  Kernels written with the plain
+// operations keep that pipe 80-85% busy, so their time is their count of FP64 instructions, and
+// 40-odd FP32 and integer instructions run in the shadow of each.  The helpers here therefore
+// form everything that need not be an FP64 instruction with FP32 and integer ones (which leaves
+// the step's three kernels at 55 to 80% of the pipe on meshes that fill the GPU, the reverse step's
+// faces at 75%):
 //   * the reciprocal (square root) seeds: FP32 approximation of the operand's leading 24
 //     bits, one Newton-Raphson step carried as a float pair with the operand's next 23
 //     bits (2^-44 relative), a second one in 64-bit fixed point, rounded to a double:
